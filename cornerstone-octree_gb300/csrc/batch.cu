@@ -79,7 +79,7 @@ struct Batch final : BatchBase
     DevBuf setOff, keyParams, geoParams, buckets, initTree, initOff, roots, leafBegin;
     DevBuf buildWs, leaves, counts, layout;
     DevBuf prefixes, childOffsets, parents, levelRange, i2l, l2i, linkWs, centers, sizes;
-    DevBuf nbPrepWs, pout, nb, nc;
+    DevBuf nbPrepWs, pnode, nb, nc;
     int capacity = 0;
     size_t n     = 0;
     cs_batch_result last{};
@@ -94,7 +94,7 @@ struct Batch final : BatchBase
                                 &sortWs, &errWords,
                                 &setOff, &keyParams, &geoParams, &buckets, &initTree, &initOff, &roots, &leafBegin,
                                 &buildWs, &leaves, &counts, &layout, &prefixes, &childOffsets, &parents, &levelRange,
-                                &i2l, &l2i, &linkWs, &centers, &sizes, &nbPrepWs, &pout, &nb, &nc})
+                                &i2l, &l2i, &linkWs, &centers, &sizes, &nbPrepWs, &pnode, &nb, &nc})
             t += b->bytes;
         return t;
     }
@@ -267,7 +267,7 @@ struct Batch final : BatchBase
         {
             if ((rc = nb.ensure(std::max<size_t>(1, n * cfg.ngmax) * sizeof(uint32_t)))) return rc;
             if ((rc = nbPrepWs.ensure(nbPrepBytes(0, N)))) return rc;
-            if ((rc = pout.ensure(n))) return rc;
+            if ((rc = pnode.ensure(n * sizeof(uint32_t)))) return rc;
             NbPrep prep{};
             prep.cmax = cmax;
             prep.phi  = shadows ? shadowHi.as<float4>() : nullptr;
@@ -278,17 +278,16 @@ struct Batch final : BatchBase
                 return rc;
             if ((rc = nbMarkOutside<T>(s, xs.as<T>(), ys.as<T>(), zs.as<T>(), prep.phi, centers.as<T>(), sizes.as<T>(),
                                        childOffsets.as<int32_t>(), i2l.as<int32_t>(), layout.as<uint32_t>(), N, prep,
-                                       pout.as<uint8_t>())))
+                                       pnode.as<uint32_t>())))
                 return rc;
-            prep.pout = pout.as<uint8_t>();
+            prep.pnode = pnode.as<uint32_t>();
             cs_box open{{0, 0, 0}, {1, 1, 1}, {CS_OPEN, CS_OPEN, CS_OPEN}};
             cs_ns_view nv{L, N, childOffsets.as<int32_t>(), parents.as<int32_t>(), i2l.as<int32_t>(),
                           layout.as<uint32_t>(), centers.p, sizes.p, cfg.search_ext};
             NbArgs<T> a  = makeNbArgs<T>(xs.as<T>(), ys.as<T>(), zs.as<T>(), hs.as<T>(), 0, uint32_t(n), open, nv,
                                          cfg.ngmax, nb.as<uint32_t>(), nc.as<uint32_t>());
             a.errWord      = err + 3;
-            a.groupSize    = tuning.nb_group;
-            a.byTargetCost = tuning.nb_by_target_cost;
+            a.groupSize = tuning.nb_group;
             a.setOffsets   = setOff.as<uint32_t>();
             a.setRoots   = roots.as<int32_t>();
             a.numSets    = S;

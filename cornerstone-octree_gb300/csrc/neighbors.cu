@@ -6,18 +6,11 @@
 // storing the first ngmax of them in visiting order; the count is not capped. Leaves are met in SFC order, so the
 // stored neighbours are the first ngmax in ascending j among those on leaves whose whole root path passed the test.
 //
-// Main kernel (findNeighborsGroupKernel): one warp serves 32 consecutive targets and walks the tree ONCE for all of
-// them, depth first with an explicit stack of (child offset or leaf code, lane mask) in shared memory, lowest child
-// first. A child is pushed when it can hold a neighbour of some lane: lane l tests child l % 8 against the bounding
-// box and bounding sphere of its sub-group of 8 targets (l / 8), and a child carries the lanes of the sub-groups that
-// may reach it; a warp whose targets are spread far apart, or that has already expanded many nodes, tests each child
-// per lane instead. At a leaf, each lane decides with a conservative box test whether it needs the leaf; the leaf's
-// candidates come 32 at a time, and a batch is tested either per lane (each needing lane against all staged
-// candidates, two per packed FP32 instruction, comparison signs appended to bit masks) or, when few lanes need it,
-// per target (lanes hold the candidates, the warp loops over the needing targets with two ballots each); both give
-// the same masks. The targets per warp (32, 16, 8) and the switch between the two loops are runtime tuning
-// (NbArgs::groupSize, byTargetCost). Visiting superset leaves is harmless as long as the final decision equals the
-// reference's, which depends on the whole root path (next paragraph).
+// Main kernel (findNeighborsTileKernel, neighbor_tiles.cuh): one warp serves 32 consecutive targets, walks the tree once
+// for all of them, packs the candidates near them into tiles of 32 and tests a tile against the 32 targets with tensor
+// core products. findNeighborsGroupKernel serves the smaller groups that a caller may ask for (16 or 8 targets per warp,
+// 2 or 4 lanes per target; NbArgs::groupSize). Visiting superset leaves is harmless as long as the final decision equals
+// the reference's, which depends on the whole root path (next paragraph).
 //
 // Path safety. A candidate at distance^2 d2 < r2 is counted by the reference only if each ancestor of its leaf passed
 // the cell test. Every ancestor contains the candidate's key cell, so minDistance(x_i, ancestor) <= |x_j - x_i| up to
@@ -28,11 +21,9 @@
 // d2 < min(r2, Tsafe) are accepted outright; the rare ones in [Tsafe, r2) (only when ext < 1 + O(kappa)) walk the
 // ancestor chain explicitly through parents[] with the reference's cell test.
 //
-// Arithmetic. T = float decides with the reference's expressions in round-to-nearest intrinsics (no contraction). The
-// one-target-per-lane loops first evaluate the squared distance of the reference's own differences with packed FMAs,
-// fma(dz, dz, fma(dy, dy, dx dx)); it and the reference's RN(RN(RN(dx dx) + RN(dy dy)) + RN(dz dz)) are each within
-// 3 u d2 + 3 2^-150 of the exact sum (u = 2^-24), so below min(r2, Tsafe) (1 - 8 u) - 2^-146 the pair is a path-safe
-// neighbour, from r2 (1 + 8 u) + 2^-146 on it is not, and only the band between is evaluated again unfused.
+// Arithmetic. T = float decides with the reference's expressions in round-to-nearest intrinsics (no contraction); the
+// tiles first evaluate FP32 distances in a frame, with the bounds below (the rounding of the reference's own FP32 sums,
+// 5 u d2, is inside their 24 eps), and only the band around r2 is evaluated again unfused.
 // T = double (GB300 has little FP64 throughput) first evaluates each test in FP32 on coordinates relative to a
 // per-warp reference point P, with a proven bound on the difference to the FP64 result:
 //   candidate  a_j = fl((xhi_j - P) + xlo_j)  (x = xhi + xlo, two floats),  target b_i = fl(x_i - P)
@@ -52,6 +43,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <cuda_fp16.h>
 #include <type_traits>
 
 namespace csg
@@ -428,19 +420,10 @@ __global__ void __launch_bounds__(NB_THREADS) findNeighborsKernel(NbArgs<T> a, N
 // pending siblings on each of the levels 1..d and pushes at most 8 children: 7 * 20 + 8 = 148 entries. The overflow
 // check stays, and the shared memory saved goes to L1 (the kernel's node records and candidates).
 constexpr int NBG_STACK = 152;
-// resident blocks of 4 warps per SM: 64 registers per thread (a few spilled to the L1-cached stack); 7 and 9 measured
-// slower on the 16M Plummer search
+// resident blocks of 4 warps per SM: 64 registers per thread
 #ifndef NBG_MIN_BLOCKS
 #define NBG_MIN_BLOCKS 8
 #endif
-// leaves merged into one candidate range at most (one target per lane), and the longest merged range
-#ifndef NBG_MERGE
-#define NBG_MERGE 8
-#endif
-#ifndef NBG_MERGE_SPAN
-#define NBG_MERGE_SPAN 32
-#endif
-
 // exact decision of a pair in the ambiguous band (T = double): d2 < r2 and the reference's path condition
 __device__ __noinline__ bool pairDecideF64(double xi, double yi, double zi, double r2, double cellR2, double kappa,
                                            const double* x, const double* y, const double* z, uint32_t j, int leafNode,
@@ -576,11 +559,11 @@ __device__ __forceinline__ float warpMinF(float v)
     return v;
 }
 
-template<class T, bool Stats, int G>
+template<class T, int G>
 __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroupKernel(NbArgs<T> a, NbPrep prep)
 {
     // G targets per warp; the 32 / G lanes of one target test consecutive candidates side by side
-    static_assert(G == 8 || G == 16 || G == 32, "targets per warp");
+    static_assert(G == 8 || G == 16, "targets per warp");
     constexpr int S      = 32 / G;
     constexpr bool F64   = std::is_same_v<T, double>;
     constexpr float EPS  = EPS32;
@@ -592,14 +575,6 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
     // out = 1 when it holds particles outside its box
     __shared__ int2 sStack[NB_WARPS][NBG_STACK];
     __shared__ float4 sCand[NB_WARPS][32];
-    // S == 1: the staged candidates as separate x, y, z rows, read four at a time (two float2 pairs)
-    __shared__ __align__(16) float sCx[NB_WARPS][32], sCy[NB_WARPS][32], sCz[NB_WARPS][32];
-    // S == 1: each lane's target for the by-target loop: negated frame coordinates and -Tin, and -Tup
-    __shared__ float4 sTgtA[NB_WARPS][32];
-    __shared__ float sTgtB[NB_WARPS][32];
-    // S == 1: leaves merged into one candidate range (their particle ranges adjoin): end of each range and its node
-    __shared__ int2 sMerge[NB_WARPS][NBG_MERGE];
-
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = lane % G, s = lane / G;
     const size_t wid   = size_t(blockIdx.x) * NB_WARPS + warp;
@@ -660,7 +635,10 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
         cHi  = __double2float_ru(cellR2);
     }
     else { r2lo = r2hi = r2; cLo = cHi = cellR2; }
-    float rr = __fsqrt_ru(r2hi);
+    // nodes within the cell radius are visited too where it is the larger one: a particle outside its leaf's box can be
+    // within r although the box is not
+    const float visit2 = a.ext > 1.f ? fmaxf(r2hi, cHi) : r2hi;
+    float rr = __fsqrt_ru(r2hi), vr = __fsqrt_ru(visit2);
     // path-safe threshold (lower bound)
     float tsafe = __fadd_rd(__fadd_rd(__fmul_rd(cLo, 1.f - RHO), -__fmul_ru(__fmul_ru(4.f, kappa), __fsqrt_ru(cHi))),
                             -__fmul_ru(__fmul_ru(4.f, kappa), kappa));
@@ -681,49 +659,28 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
     float gc[3], gh[3], gR2 = 0.f, rmax = 0.f;
     unsigned activeMask = 0;
     int rootNode        = 0;
-    // With one target per lane (S == 1) the bounds are those of the lane's sub-group of 8 consecutive targets (lanes
-    // 8g .. 8g + 7), so that a node is only carried for the sub-groups that can reach it; otherwise the whole warp's.
-    constexpr bool SUB = S == 1;
-    auto segMin = [&](float v) {
-        if constexpr (SUB)
-        {
-            for (int o = 4; o > 0; o >>= 1)
-                v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-            return v;
-        }
-        else return warpMinF(v);
-    };
-    auto segMax = [&](float v) {
-        if constexpr (SUB)
-        {
-            for (int o = 4; o > 0; o >>= 1)
-                v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-            return v;
-        }
-        else return warpMaxF(v);
-    };
     auto groupBounds = [&](bool inPass) {
-        float rad = __fmul_ru(rr, 1.f + 64 * EPS);
+        float rad = __fmul_ru(vr, 1.f + 64 * EPS);
 #pragma unroll
         for (int k = 0; k < 3; ++k)
         {
             float slack = __fmaf_ru(2 * EPS, fabsf(b[k]), delta);
             float lo    = inPass ? __fsub_rd(__fsub_rd(b[k], rad), slack) : INFINITY;
             float hi    = inPass ? __fadd_ru(__fadd_ru(b[k], rad), slack) : -INFINITY;
-            lo          = segMin(lo);
-            hi          = segMax(hi);
+            lo          = warpMinF(lo);
+            hi          = warpMaxF(hi);
             gc[k]       = 0.5f * (lo + hi);
             gh[k]       = __fmul_ru(__fsub_ru(hi, lo), 0.5f);
         }
         // bounding sphere around the box centre gc: every point of every lane's sphere is within gR of gc, so it cuts
         // the corners of the box (which matter where the density rises steeply, e.g. towards a Plummer core)
         activeMask = __ballot_sync(0xffffffffu, inPass);
-        rmax       = segMax(inPass ? rr : 0.f);
+        rmax       = warpMaxF(inPass ? rr : 0.f);
         float e0 = b[0] - gc[0], e1 = b[1] - gc[1], e2 = b[2] - gc[2];
         float dc = __fsqrt_ru(__fmaf_ru(e2, e2, __fmaf_ru(e1, e1, __fmul_ru(e0, e0))));
         float sl = __fmaf_ru(2 * EPS, fmaxf(fabsf(b[0]), fmaxf(fabsf(b[1]), fabsf(b[2]))), delta);
-        float gr = inPass ? __fadd_ru(__fadd_ru(__fmul_ru(dc, 1.f + 8 * EPS), __fmul_ru(rr, 1.f + 64 * EPS)), sl) : 0.f;
-        gr       = segMax(gr);
+        float gr = inPass ? __fadd_ru(__fadd_ru(__fmul_ru(dc, 1.f + 8 * EPS), __fmul_ru(vr, 1.f + 64 * EPS)), sl) : 0.f;
+        gr       = warpMaxF(gr);
         gR2      = __fmul_ru(gr, gr);
     };
 
@@ -735,16 +692,6 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
 #pragma unroll
     for (int q = 0; q < S; ++q)
         tmask |= 1u << (t + q * G);
-    unsigned long long stLeaves = 0, stCand = 0, stNodes = 0, stPair = 0, stExact = 0;
-    // cost model of the candidate batches (lane 0): steps of the lane-per-target loop, needing lanes, the cheaper of
-    // 11 instructions per step and 20 per needing lane, batches, cycles spent in the batches
-    unsigned long long stSteps = 0, stNeed = 0, stMinCost = 0, stBatches = 0, stCandCyc = 0;
-    // cycles in leaf visits (box test, staging and batches) and leaf visits no lane needed
-    unsigned long long stLeafCyc = 0, stLeafIdle = 0;
-    // output loop shapes per batch: the most hits of one lane, lanes with hits, rounds of 32 hits
-    unsigned long long stOutMax = 0, stOutLanes = 0, stOutRounds = 0;
-    unsigned long long stPathWalks = 0; // exact path walks to leaves holding particles outside their box
-
     // node box in the warp frame: center cc = (chi - P) + clo, half size sz
     auto frameOf = [&](float4 ch, float4 cl, float4 s4, float cc[3], float sz[3]) {
         cc[0] = __fadd_rn(__fsub_rn(ch.x, P[0]), cl.x);
@@ -754,11 +701,6 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
         sz[1] = s4.y;
         sz[2] = s4.z;
     };
-    auto nodeFrame = [&](int node, float cc[3], float sz[3]) {
-        const float4* r = prep.nrec + 3 * size_t(node);
-        frameOf(r[0], r[1], r[2], cc, sz);
-    };
-
     // conservative per-lane test: can a particle of this node lie within the search radius of x_i? (a lower
     // bound of |x_i - node box|, the box widened by the particle slack delta)
     // per axis (D - sz) - u with u = 4.5 EPS (D + sz) + 1.05 A + delta, evaluated as two FMAs with the factors
@@ -773,14 +715,8 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
             float d = fmaxf(__fmaf_rd(D, 1.f - 5 * EPS, -__fmaf_ru(sz[k], 1.f + 6 * EPS, hitC0)), 0.f);
             n2      = __fmaf_rd(d, d, n2);
         }
-        return n2 < r2hi;
+        return n2 < visit2;
     };
-    auto mayHit = [&](int node) -> bool {
-        float cc[3], sz[3];
-        nodeFrame(node, cc, sz);
-        return mayHitBox(cc, sz);
-    };
-
     // decision for one candidate of the lane's target that survived the first distance filter; outside: the
     // candidate lies outside its leaf's box (no path-safe shortcut)
     auto decide = [&](uint32_t jj, float d2, int node, bool outside) -> bool {
@@ -790,7 +726,6 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
             in = !outside && d2 < Tacc;
             if (!in)
             {
-                if constexpr (Stats) stExact++;
                 in = pairDecideF64(xi, yi, zi, r2, cellR2, double(kappa), a.x, a.y, a.z, jj, node, a.parents,
                                    a.centers, a.sizes, !outside, rootNode);
             }
@@ -800,54 +735,12 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
             in = !outside && d2 < tsafe;
             if (!in)
             {
-                if constexpr (Stats) stExact++;
                 in = pathCheckF32(float(xi), float(yi), float(zi), float(cellR2), node, a.parents,
                                   reinterpret_cast<const float*>(a.centers),
                                   reinterpret_cast<const float*>(a.sizes), rootNode);
             }
         }
         return in && jj != i;
-    };
-    // batch thresholds of the S == 1 loop: d2 < Tin is a neighbour (self aside), d2 >= Tup is not, the rest is
-    // decided by decideSlow
-    float Tin, Tup;
-    if constexpr (F64)
-    {
-        Tin = Tacc;
-        Tup = Tout;
-    }
-    else
-    {
-        // the packed FMA distance of the batch loops is within 6 u d2 + 6 2^-150 of the reference's unfused FP32
-        // value (u = 2^-24, three roundings each, subnormal results included): below Tin the pair is a path-safe
-        // neighbour, from Tup on it is not; the band between is decided exactly (decideSlow)
-        Tin = __fsub_rd(__fmul_rd(fminf(float(r2), tsafe), 1.f - 8 * EPS), 0x1p-146f);
-        Tup = __fadd_ru(__fmul_ru(float(r2), 1.f + 8 * EPS), 0x1p-146f);
-    }
-    // minus the target in the candidates' frame, as float pairs for the packed distance evaluation
-    float nbS[3];
-    if constexpr (F64)
-    {
-        nbS[0] = -b[0];
-        nbS[1] = -b[1];
-        nbS[2] = -b[2];
-    }
-    else
-    {
-        nbS[0] = -float(xi);
-        nbS[1] = -float(yi);
-        nbS[2] = -float(zi);
-    }
-    const float nTinS = -Tin, nTupS = -Tup;
-    if constexpr (S == 1)
-    {
-        sTgtA[warp][lane] = make_float4(nbS[0], nbS[1], nbS[2], nTinS);
-        sTgtB[warp][lane] = nTupS;
-        __syncwarp();
-    }
-    const TargetRef<T> tref{a.x, a.y, a.z, a.h, a.hf, a.ext, i};
-    auto decideSlow = [&](uint32_t jj, int node, bool contained) -> bool {
-        return slowPairAt<T>(tref, kappa, tsafe, jj, node, a.parents, a.centers, a.sizes, contained, rootNode);
     };
     // first filter: FP32 distance of the staged candidate; returns d2 and whether it can be a neighbour
     auto filter = [&](float4 c, float& d2) -> bool {
@@ -883,238 +776,25 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
     };
 
     // a leaf with its record r0..r2: the lanes whose sphere may reach it test its particles, 32 per batch
-    // a leaf with its record r0..r2: the lanes whose sphere may reach it test its particles, 32 per batch. With
-    // nMerged > 1 (S == 1) the following leaves of sMerge are tested with it as one range [first, lastM): needM is
-    // this lane's need of any of them
-    auto processLeaf = [&](int node, unsigned pmask, float4 recA, float4 recB, float4 recC, bool anyOut, int nMerged,
-                           uint32_t lastM, bool needM) {
-        const uint32_t first = __float_as_uint(recB.w), last = nMerged > 1 ? lastM : __float_as_uint(recC.w);
+    auto processLeaf = [&](int node, unsigned pmask, float4 recA, float4 recB, float4 recC, bool anyOut) {
+        const uint32_t first = __float_as_uint(recB.w), last = __float_as_uint(recC.w);
         // the first batch is loaded before the lanes' box test, so that the two latencies overlap
         float4 q0 = stage(first + lane, last);
         float cc[3], sz[3];
         frameOf(recA, recB, recC, cc, sz);
-        bool need     = (((pmask >> lane) & 1u) && mayHitBox(cc, sz)) || needM;
+        bool need     = ((pmask >> lane) & 1u) && mayHitBox(cc, sz);
         unsigned mask = __ballot_sync(0xffffffffu, need);
         if (mask == 0) return;
-        // a leaf holding particles outside its box: whether this lane's path to it passes the reference's cell tests.
-        // An upper bound of |x_i - box|^2 below Tsafe proves it (the ancestors contain the leaf); otherwise the path
-        // is walked once, exactly
-        bool leafPass = true;
-        if (anyOut && need)
-        {
-            float n2u = 0.f;
-#pragma unroll
-            for (int k = 0; k < 3; ++k)
-            {
-                float D = fabsf(__fsub_rn(cc[k], b[k]));
-                float u = __fmaf_ru(4.5f * EPS, D + sz[k], __fmaf_ru(1.05f, A, delta));
-                float d = fmaxf(__fadd_ru(__fsub_ru(D, sz[k]), u), 0.f);
-                n2u     = __fmaf_ru(d, d, n2u);
-            }
-            if (!(n2u < tsafe))
-            {
-                if constexpr (Stats) stPathWalks++;
-                leafPass = leafPathAt<T>(tref, node, a.parents, a.centers, a.sizes, rootNode);
-            }
-        }
-        if constexpr (Stats)
-        {
-            stLeaves++;
-            stCand += last - first;
-        }
         for (uint32_t base = first; base < last; base += 32)
         {
             float4 q = base == first ? q0 : stage(base + lane, last);
             // candidates of this batch that lie outside their leaf's box (only in marked leaves)
             const unsigned outB =
-                anyOut ? __ballot_sync(0xffffffffu, base + lane < last && prep.pout[base + lane]) : 0u;
+                anyOut ? __ballot_sync(0xffffffffu, base + lane < last && (prep.pnode[base + lane] >> 31)) : 0u;
             int cnt = int(min(32u, last - base));
-            // S == 1: few needing lanes against many candidates are cheaper with the roles swapped (lanes hold the
-            // candidates, the warp loops over the needing targets): about 19 instructions per needing target against
-            // about byTargetCost (default 7) per candidate step of the per-lane loop (steps of eight; on the 16M
-            // Plummer search the ratio 19 : 7 measured as good as any between 19 : 9 and 24 : 7)
-            const bool byTarget = S == 1 && 19 * __popc(mask) < a.byTargetCost * ((cnt + 7) & ~7);
-            if (!byTarget)
-            {
-                __syncwarp();
-                if constexpr (S == 1)
-                {
-                    sCx[warp][lane] = q.x;
-                    sCy[warp][lane] = q.y;
-                    sCz[warp][lane] = q.z;
-                }
-                else { sCand[warp][lane] = q; }
-                __syncwarp();
-            }
-            long long tc0 = 0;
-            unsigned hitsThis = 0;
-            if constexpr (Stats)
-            {
-                unsigned steps = (unsigned(cnt) + 7u) & ~7u;
-                unsigned m     = __popc(mask);
-                stSteps += steps;
-                stNeed += m;
-                stMinCost += min(11u * steps, 20u * m);
-                stBatches++;
-                tc0 = clock64();
-            }
-            if constexpr (S == 1)
-            {
-                // Bit 31 - k of inM: candidate k passes the FP32 test outright; of ambM: it is below the upper
-                // threshold. The sign of e - T (exact for the packed add) is the comparison e < T, and a funnel shift
-                // appends it to the mask, so that the candidates of a run end in order below its first one.
-                unsigned inM = 0, ambM = 0;
-                // four candidates (two packed FP32 pairs) against the target -n (negated frame coordinates) with the
-                // negated thresholds nin, nup; the expressions are those of filter()
-                auto four = [&](const float4& x4, const float4& y4, const float4& z4, const float2 n[3], float2 nin,
-                                float2 nup, unsigned& mi, unsigned& ma) {
-#pragma unroll
-                    for (int p = 0; p < 2; ++p)
-                    {
-                        float2 cx = p ? make_float2(x4.z, x4.w) : make_float2(x4.x, x4.y);
-                        float2 cy = p ? make_float2(y4.z, y4.w) : make_float2(y4.x, y4.y);
-                        float2 cz = p ? make_float2(z4.z, z4.w) : make_float2(z4.x, z4.y);
-                        float2 dx = __fadd2_rn(cx, n[0]);
-                        float2 dy = __fadd2_rn(cy, n[1]);
-                        float2 dz = __fadd2_rn(cz, n[2]);
-                        // an FP32 filter with proven margins (the thresholds): any rounding of these FMAs stays
-                        // inside them. T = float: the differences are the reference's own, and the band around r2
-                        // is decided again with its unfused expression
-                        float2 e = __fmul2_rn(dx, dx);
-                        e        = __ffma2_rn(dy, dy, e);
-                        e        = __ffma2_rn(dz, dz, e);
-                        const float2 ti = __fadd2_rn(e, nin), tu = __fadd2_rn(e, nup);
-                        mi = __funnelshift_l(__float_as_uint(ti.x), mi, 1);
-                        mi = __funnelshift_l(__float_as_uint(ti.y), mi, 1);
-                        ma = __funnelshift_l(__float_as_uint(tu.x), ma, 1);
-                        ma = __funnelshift_l(__float_as_uint(tu.y), ma, 1);
-                    }
-                };
-                const float4* vx = reinterpret_cast<const float4*>(sCx[warp]);
-                const float4* vy = reinterpret_cast<const float4*>(sCy[warp]);
-                const float4* vz = reinterpret_cast<const float4*>(sCz[warp]);
-                // the target as packed pairs (negated frame coordinates and thresholds), built per batch from scalars
-                const float2 n[3] = {make_float2(nbS[0], nbS[0]), make_float2(nbS[1], nbS[1]),
-                                     make_float2(nbS[2], nbS[2])};
-                const float2 nin = make_float2(nTinS, nTinS), nup = make_float2(nTupS, nTupS);
-                if (byTarget)
-                {
-                    // lane k holds candidate k (past the leaf's end: a point at infinity); per needing target t the
-                    // same FP32 expressions as four(), and the two signs collected by ballots (bit k: candidate k)
-                    unsigned mm = mask, bi = 0, ba = 0;
-                    while (mm)
-                    {
-                        const int t = __ffs(mm) - 1;
-                        mm &= mm - 1;
-                        const float4 tg = sTgtA[warp][t];
-                        const float tup = sTgtB[warp][t];
-                        const float dx = __fadd_rn(q.x, tg.x), dy = __fadd_rn(q.y, tg.y), dz = __fadd_rn(q.z, tg.z);
-                        float e;
-                        e = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-                        const unsigned mi = __ballot_sync(0xffffffffu, __float_as_int(__fadd_rn(e, tg.w)) < 0);
-                        const unsigned ma = __ballot_sync(0xffffffffu, __float_as_int(__fadd_rn(e, tup)) < 0);
-                        if (lane == t)
-                        {
-                            bi = mi;
-                            ba = ma;
-                        }
-                    }
-                    inM  = __brev(bi);
-                    ambM = __brev(ba);
-                }
-                else if (need)
-                {
-                    // eight independent distance chains per step; the staged points past the leaf's end never pass
-                    int steps = 0;
-                    for (int k0 = 0; k0 < cnt; k0 += 8, steps += 8)
-                    {
-                        const int v = k0 >> 2;
-                        four(vx[v], vy[v], vz[v], n, nin, nup, inM, ambM);
-                        four(vx[v + 1], vy[v + 1], vz[v + 1], n, nin, nup, inM, ambM);
-                    }
-                    if (steps < 32)
-                    {
-                        inM <<= 32 - steps;
-                        ambM <<= 32 - steps;
-                    }
-                }
-                if (need)
-                {
-                    ambM &= ~inM;
-                    const unsigned outR = __brev(outB); // bit 31 - k: candidate k lies outside its leaf's box
-                    // candidates outside their leaf's box: no path-safe shortcut; a neighbour iff within r and the
-                    // lane's path to the leaf passes. Below Tin the FP32 bound already proves d2 < r2; the band
-                    // [Tin, Tup) is decided exactly
-                    const unsigned fIn = inM & outR, fAmb = ambM & outR;
-                    inM &= ~outR;
-                    ambM &= ~outR;
-                    if (leafPass)
-                    {
-                        inM |= fIn;
-                        // group warps have no periodic sphere
-                        unsigned f = fAmb;
-                        while (f)
-                        {
-                            int k = __clz(f);
-                            f &= ~(0x80000000u >> k);
-                            if (pairWithinAt(tref, base + k)) inM |= 0x80000000u >> k;
-                        }
-                    }
-                    if constexpr (Stats)
-                    {
-                        stPair += cnt;
-                        stExact += __popc(ambM);
-                    }
-                    while (ambM)
-                    {
-                        int k = __clz(ambM);
-                        ambM &= ~(0x80000000u >> k);
-                        int kn = node;
-                        if (nMerged > 1)
-                            for (int m = 0; m < nMerged; ++m)
-                                if (base + k < uint32_t(sMerge[warp][m].x))
-                                {
-                                    kn = sMerge[warp][m].y;
-                                    break;
-                                }
-                        if (decideSlow(base + k, kn, true)) inM |= 0x80000000u >> k;
-                    }
-                    if (i >= base && i - base < 32u) inM &= ~(0x80000000u >> (i - base));
-                    if constexpr (Stats) hitsThis = __popc(inM);
-                    // the hits in ascending candidate order; while the row has room for all of them (the common
-                    // case) two per round, without a bound check per hit
-                    const unsigned nh = __popc(inM);
-                    if (nc + nh <= ngmax)
-                    {
-                        uint32_t* p = myNb + nc;
-                        while (inM)
-                        {
-                            const int k1 = __clz(inM);
-                            inM ^= 0x80000000u >> k1;
-                            p[0] = base + k1;
-                            if (inM)
-                            {
-                                const int k2 = __clz(inM);
-                                inM ^= 0x80000000u >> k2;
-                                p[1] = base + k2;
-                            }
-                            p += 2;
-                        }
-                        nc += nh;
-                    }
-                    else
-                    {
-                        while (inM)
-                        {
-                            int k = __clz(inM);
-                            inM &= ~(0x80000000u >> k);
-                            if (nc < ngmax) myNb[nc] = base + k;
-                            nc++;
-                        }
-                    }
-                }
-            }
-            else
+            __syncwarp();
+            sCand[warp][lane] = q;
+            __syncwarp();
             {
                 // lane (t, s) tests candidate k0 + s for target t; a ballot keeps each target's hits in order
                 for (int k0 = 0; k0 < cnt; k0 += S)
@@ -1125,7 +805,6 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
                     if (need && k < cnt)
                     {
                         float e;
-                        if constexpr (Stats) stPair++;
                         in = filter(sCand[warp][k], e) && decide(jj, e, node, (outB >> k) & 1u);
                     }
                     unsigned hits = __ballot_sync(0xffffffffu, in);
@@ -1138,16 +817,6 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
                     nc += __popc(mine);
                 }
             }
-            if constexpr (Stats)
-            {
-                __syncwarp();
-                stCandCyc += (unsigned long long)(clock64() - tc0);
-                const unsigned mx  = __reduce_max_sync(0xffffffffu, hitsThis);
-                const unsigned tot = __reduce_add_sync(0xffffffffu, hitsThis);
-                stOutMax += mx;
-                stOutLanes += __popc(__ballot_sync(0xffffffffu, hitsThis != 0));
-                stOutRounds += (tot + 31) / 32;
-            }
         }
     };
 
@@ -1159,10 +828,8 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
     constexpr int LOOSE_AFTER = 96;
     bool loose                = false;
     int expansions            = 0;
-    long long t0              = Stats ? clock64() : 0;
     // absolute part of the child test's margin: the rounding terms and the float centre's missing low part
     const float childMargin = __fadd_ru(__fmaf_ru(4 * EPS * EPS, C, delta), __fmul_ru(EPS, C));
-    float rminW               = Stats ? warpMinF(active ? rr : INFINITY) : 0.f;
     int2* stack               = sStack[warp];
     auto entryCode            = [](int node, int c0) { return c0 > 0 ? c0 : -(2 * node + (c0 < 0 ? 1 : 0)) - 1; };
 
@@ -1208,67 +875,22 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
             const bool out = (-c0 - 1) & 1;
             const float4* rec = prep.nrec + 3 * size_t(node);
             float4 recA = rec[0], recB = rec[1], recC = rec[2];
-            long long tl0 = Stats ? clock64() : 0;
-            unsigned long long before = stLeaves;
-            // S == 1: the next leaves on the stack whose particles continue this leaf's range (siblings and cousins
-            // met consecutively in SFC order) join its candidate range while it stays within NBG_MERGE_SPAN
-            // particles; a
-            // lane then tests all of them, which changes no decision (a candidate outside a lane's sphere fails its
-            // distance test), and the batch overhead is paid once. Leaves holding particles outside their box stay alone
-            int nMerged    = 1;
-            uint32_t lastM = __float_as_uint(recC.w);
-            bool needM     = false;
-            if constexpr (S == 1)
-            {
-                const uint32_t first = __float_as_uint(recB.w);
-                while (!out && top > 0 && nMerged < NBG_MERGE && lastM - first < unsigned(NBG_MERGE_SPAN))
-                {
-                    const int2 nx = stack[top - 1];
-                    if (nx.x > 0 || ((-nx.x - 1) & 1)) break; // an internal node, or a leaf with outside particles
-                    const int nnode    = (-nx.x - 1) >> 1;
-                    const float4* nrc  = prep.nrec + 3 * size_t(nnode);
-                    const float4 nB = nrc[1], nC = nrc[2];
-                    if (__float_as_uint(nB.w) != lastM || __float_as_uint(nC.w) - first > unsigned(NBG_MERGE_SPAN))
-                        break;
-                    const float4 nA = nrc[0];
-                    float cc[3], sz[3];
-                    frameOf(nA, nB, nC, cc, sz);
-                    needM = needM || (((unsigned(nx.y) >> lane) & 1u) && mayHitBox(cc, sz));
-                    if (lane == 0)
-                    {
-                        if (nMerged == 1) sMerge[warp][0] = make_int2(int(lastM), node);
-                        sMerge[warp][nMerged] = make_int2(int(__float_as_uint(nC.w)), nnode);
-                    }
-                    lastM = __float_as_uint(nC.w);
-                    ++nMerged;
-                    --top;
-                }
-                if (nMerged > 1) __syncwarp();
-            }
-            processLeaf(node, pmask, recA, recB, recC, out, nMerged, lastM, needM);
-            if constexpr (Stats)
-            {
-                stLeafCyc += (unsigned long long)(clock64() - tl0);
-                stLeafIdle += stLeaves == before;
-            }
+            processLeaf(node, pmask, recA, recB, recC, out);
             continue;
         }
-        if constexpr (Stats) stNodes++;
         if (++expansions > LOOSE_AFTER) loose = true;
         bool ok         = false;
         unsigned cmask  = pmask; // lanes alive in the accepted child (this lane's child when lane < 8)
         int childC0     = 0;     // child offset of this lane's child (lane < 8)
         if (!loose)
         {
-            // lane l tests child l & 7 against its sub-group's bounds (every lane of one sub-group tests the 8
-            // children; S > 1: lanes 0-7 against the warp's bounds)
-            const int cidx = SUB ? (lane & 7) : lane;
-            bool hit       = false;
-            if (SUB || lane < 8)
+            // lanes 0-7 test the eight children against the warp's bounds
+            bool hit = false;
+            if (lane < 8)
             {
                 // the child's centre in the frame from its float centre alone (the low part, at most EPS C, is
                 // covered by childMargin), so one load of its record is saved
-                const float4* r = prep.nrec + 3 * size_t(c0 + cidx);
+                const float4* r = prep.nrec + 3 * size_t(c0 + lane);
                 const float4 rA = r[0], rC = r[2];
                 const float cc[3] = {__fsub_rn(rA.x, P[0]), __fsub_rn(rA.y, P[1]), __fsub_rn(rA.z, P[2])};
                 const float sz[3] = {rC.x, rC.y, rC.z};
@@ -1288,14 +910,7 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
                 }
                 hit = hit && dist2 <= gR2;
             }
-            if constexpr (SUB)
-            {
-                // bit 8g + c: sub-group g may reach child c; the lanes of child c are those sub-groups' alive lanes
-                const unsigned m32 = __ballot_sync(0xffffffffu, hit);
-                cmask              = pmask & (((m32 >> cidx) & 0x01010101u) * 0xFFu);
-                ok                 = lane < 8 && cmask != 0;
-            }
-            else { ok = hit; }
+            ok = hit;
         }
         else
         {
@@ -1335,59 +950,9 @@ __global__ void __launch_bounds__(NB_THREADS, NBG_MIN_BLOCKS) findNeighborsGroup
     if (!a.numSets || passSet >= lastSet) break;
     } // passes
     if (active && s == 0) a.nc[i - a.first] = nc;
-    if constexpr (Stats)
-    {
-        {
-            unsigned long long x = stPathWalks;
-            for (int o = 16; o > 0; o >>= 1)
-                x += __shfl_xor_sync(0xffffffffu, x, o);
-            if (lane == 0) atomicAdd(a.stats + 31, x);
-        }
-        unsigned long long v[5] = {stPair, stExact, stLeaves, stCand, stNodes};
-#pragma unroll
-        for (int k = 0; k < 5; ++k)
-        {
-            unsigned long long x = v[k];
-            if (k >= 2) x = lane == 0 ? x : 0;
-            for (int o = 16; o > 0; o >>= 1)
-                x += __shfl_xor_sync(0xffffffffu, x, o);
-            // same slots as findNeighborsKernel: [2] pair tests, [3] exact, [4] leaves, [5] candidates, [6] nodes
-            if (lane == 0) atomicAdd(a.stats + 2 + k, x);
-        }
-        if (lane == 0)
-        {
-            atomicAdd(a.stats + 20, stSteps);
-            atomicAdd(a.stats + 21, stNeed);
-            atomicAdd(a.stats + 22, stMinCost);
-            atomicAdd(a.stats + 23, stBatches);
-            atomicAdd(a.stats + 24, stCandCyc);
-            atomicAdd(a.stats + 25, (unsigned long long)(clock64() - t0));
-            atomicAdd(a.stats + 26, stLeafCyc);
-            atomicAdd(a.stats + 27, stLeafIdle);
-            atomicAdd(a.stats + 28, stOutMax);
-            atomicAdd(a.stats + 29, stOutLanes);
-            atomicAdd(a.stats + 30, stOutRounds);
-            atomicAdd(a.stats + 7, 1ull);
-            // slowest warp: [8] cycles, [9] its expansions, [10] leaves, [11] candidates, [12] loose flag,
-            // [13] its first target; [14] number of loose warps
-            unsigned long long cyc = (unsigned long long)(clock64() - t0);
-            if (atomicMax(a.stats + 8, cyc) < cyc)
-            {
-                a.stats[9]  = stNodes;
-                a.stats[10] = stLeaves;
-                a.stats[11] = stCand;
-                a.stats[12] = loose;
-                a.stats[13] = base0;
-                a.stats[15] = __float_as_uint(rmax);
-                a.stats[16] = __float_as_uint(__fsqrt_ru(gR2));
-                a.stats[17] = __float_as_uint(fmaxf(gh[0], fmaxf(gh[1], gh[2])));
-                a.stats[18] = __float_as_uint(rminW);
-                a.stats[19] = __float_as_uint(C);
-            }
-            if (loose) atomicAdd(a.stats + 14, 1ull);
-        }
-    }
 }
+
+#include "neighbor_tiles.cuh"
 
 // float shadows of the FP64 particle coordinates and node boxes, and the magnitude bound C
 __global__ void prepParticlesKernel(const double* __restrict__ x, const double* __restrict__ y,
@@ -1503,7 +1068,7 @@ template<class T>
 __global__ void markOutsideKernel(const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ z,
                                   const float4* __restrict__ phi, const T* __restrict__ centers,
                                   const T* __restrict__ sizes, int Nhost, const int* Ldev, float4* __restrict__ nrec,
-                                  uint8_t* __restrict__ pout)
+                                  uint32_t* __restrict__ pnode)
 {
     const size_t gtid = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int sub = int(gtid % MARK_LANES), lane = threadIdx.x & 31;
@@ -1559,7 +1124,7 @@ __global__ void markOutsideKernel(const T* __restrict__ x, const T* __restrict__
                 o = RN<T>::abs_(RN<T>::sub(x[j], c[0])) > s[0] || RN<T>::abs_(RN<T>::sub(y[j], c[1])) > s[1] ||
                     RN<T>::abs_(RN<T>::sub(z[j], c[2])) > s[2];
             }
-            pout[j] = o ? 1 : 0;
+            pnode[j] = uint32_t(node) | (o ? 0x80000000u : 0u);
         }
         any |= (__ballot_sync(0xffffffffu, o) & segMask) != 0u;
     }
@@ -1569,7 +1134,7 @@ __global__ void markOutsideKernel(const T* __restrict__ x, const T* __restrict__
 template<class T>
 int nbMarkOutside(cudaStream_t s, const T* x, const T* y, const T* z, const float4* phi, const T* centers,
                   const T* sizes, const int32_t* childOffsets, const int32_t* i2l, const uint32_t* layout,
-                  int numNodes, const NbPrep& prep, uint8_t* pout, const int* Ldev)
+                  int numNodes, const NbPrep& prep, uint32_t* pnode, const int* Ldev)
 {
     if (numNodes <= 0) return CS_OK;
     if (std::is_same_v<T, double> && !phi)
@@ -1578,17 +1143,17 @@ int nbMarkOutside(cudaStream_t s, const T* x, const T* y, const T* z, const floa
         return CS_ERR_INVALID;
     }
     markOutsideKernel<T><<<iceil(size_t(numNodes) * MARK_LANES, 256), 256, 0, s>>>(
-        x, y, z, phi, centers, sizes, numNodes, Ldev, const_cast<float4*>(prep.nrec), pout);
+        x, y, z, phi, centers, sizes, numNodes, Ldev, const_cast<float4*>(prep.nrec), pnode);
     CSG_CHECK_LAUNCH();
     return CS_OK;
 }
 
 template int nbMarkOutside<float>(cudaStream_t, const float*, const float*, const float*, const float4*,
                                   const float*, const float*, const int32_t*, const int32_t*, const uint32_t*, int,
-                                  const NbPrep&, uint8_t*, const int*);
+                                  const NbPrep&, uint32_t*, const int*);
 template int nbMarkOutside<double>(cudaStream_t, const double*, const double*, const double*, const float4*,
                                    const double*, const double*, const int32_t*, const int32_t*, const uint32_t*, int,
-                                   const NbPrep&, uint8_t*, const int*);
+                                   const NbPrep&, uint32_t*, const int*);
 
 size_t nbPrepBytes(size_t n, int numNodes)
 {
@@ -1597,7 +1162,7 @@ size_t nbPrepBytes(size_t n, int numNodes)
     ar.take<float4>(n);
     ar.take<float4>(3 * size_t(numNodes));
     ar.take<float>(1);
-    ar.take<uint8_t>(n);
+    ar.take<uint32_t>(n);
     return ar.size + 256;
 }
 
@@ -1612,7 +1177,7 @@ int nbPrepare(cudaStream_t s, const T* x, const T* y, const T* z, size_t n, cons
     float4* plo  = ar.take<float4>(F64 ? n : 0);
     float4* nrec  = ar.take<float4>(3 * size_t(numNodes));
     float* cmax   = ar.take<float>(1);
-    uint8_t* pout = ar.take<uint8_t>(n);
+    uint32_t* pnode = ar.take<uint32_t>(n);
     if (!ar.ok())
     {
         setLastError("find neighbors: workspace too small");
@@ -1636,9 +1201,9 @@ int nbPrepare(cudaStream_t s, const T* x, const T* y, const T* z, size_t n, cons
                                                   cmax);
     }
     CSG_CHECK_LAUNCH();
-    *prep  = NbPrep{phi, plo, nrec, cmax, pout};
+    *prep  = NbPrep{phi, plo, nrec, cmax, pnode};
     int rc = nbMarkOutside<T>(s, x, y, z, F64 ? phi : nullptr, centers, sizes, childOffsets, i2l, layout, numNodes,
-                              *prep, pout);
+                              *prep, pnode);
     return rc;
 }
 
@@ -1683,10 +1248,10 @@ template int nbPrepare<double>(cudaStream_t, const double*, const double*, const
                                const double*, const int32_t*, const int32_t*, const uint32_t*, int, void*, size_t,
                                NbPrep*);
 
-// The smallest shared-memory carveout that keeps NBG_MIN_BLOCKS blocks of the kernel resident (1 KB per block is
+// The smallest shared-memory carveout that keeps MinBlocks blocks of the kernel resident (1 KB per block is
 // reserved by the runtime), so that the rest of the unified L1 / shared storage caches node records and candidates.
 // Set once per kernel.
-template<auto Kernel>
+template<auto Kernel, int MinBlocks>
 static void preferL1()
 {
     static const bool done = [] {
@@ -1699,7 +1264,7 @@ static void preferL1()
             (void)cudaGetLastError();
             return false;
         }
-        const size_t need = size_t(NBG_MIN_BLOCKS) * (fa.sharedSizeBytes + 1024);
+        const size_t need = size_t(MinBlocks) * (fa.sharedSizeBytes + 1024);
         const int pct     = int(std::min<size_t>(100, (need * 100 + size_t(smemSM) - 1) / size_t(smemSM) + 1));
         if (cudaFuncSetAttribute(Kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct) != cudaSuccess)
             (void)cudaGetLastError();
@@ -1708,11 +1273,11 @@ static void preferL1()
     (void)done;
 }
 
-template<class T, bool Stats, int G>
+template<auto Kernel, int MinBlocks, class T>
 static void launchGroup(unsigned gblk, cudaStream_t s, const NbArgs<T>& a, const NbPrep& prep)
 {
-    preferL1<findNeighborsGroupKernel<T, Stats, G>>();
-    findNeighborsGroupKernel<T, Stats, G><<<gblk, NB_THREADS, 0, s>>>(a, prep);
+    preferL1<Kernel, MinBlocks>();
+    Kernel<<<gblk, NB_THREADS, 0, s>>>(a, prep);
 }
 
 template<class T>
@@ -1723,24 +1288,13 @@ int findNeighbors(cudaStream_t s, const NbArgs<T>& a0, const NbPrep& prep)
     size_t blocks = (warps + NB_WARPS - 1) / NB_WARPS;
     NbArgs<T> a   = a0;
     a.pathOnlyPbcWarps = 0;
-    int G = a.groupSize == 8 || a.groupSize == 16 || a.groupSize == 32 ? a.groupSize : 32;
-    size_t gwarps  = (size_t(a.last - a.first) + G - 1) / G;
-    unsigned gblk  = unsigned((gwarps + NB_WARPS - 1) / NB_WARPS);
-    if (G == 8)
-    {
-        if (a.stats) launchGroup<T, true, 8>(gblk, s, a, prep);
-        else launchGroup<T, false, 8>(gblk, s, a, prep);
-    }
-    else if (G == 16)
-    {
-        if (a.stats) launchGroup<T, true, 16>(gblk, s, a, prep);
-        else launchGroup<T, false, 16>(gblk, s, a, prep);
-    }
-    else
-    {
-        if (a.stats) launchGroup<T, true, 32>(gblk, s, a, prep);
-        else launchGroup<T, false, 32>(gblk, s, a, prep);
-    }
+    const int G = a.groupSize == 8 || a.groupSize == 16 ? a.groupSize : 32;
+    const size_t gwarps = (size_t(a.last - a.first) + G - 1) / G;
+    const unsigned gblk = unsigned((gwarps + NB_WARPS - 1) / NB_WARPS);
+    if (G == 8) launchGroup<findNeighborsGroupKernel<T, 8>, NBG_MIN_BLOCKS>(gblk, s, a, prep);
+    else if (G == 16) launchGroup<findNeighborsGroupKernel<T, 16>, NBG_MIN_BLOCKS>(gblk, s, a, prep);
+    else if (a.stats) launchGroup<findNeighborsTileKernel<T, true>, NT_MIN_BLOCKS>(gblk, s, a, prep);
+    else launchGroup<findNeighborsTileKernel<T, false>, NT_MIN_BLOCKS>(gblk, s, a, prep);
     CSG_CHECK_LAUNCH();
     if (a.anyPbc)
     {

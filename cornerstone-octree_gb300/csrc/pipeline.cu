@@ -36,7 +36,7 @@ struct Pipeline final : PipelineBase
     DevBuf keys, keysAlt, order, orderAlt;
     DevBuf xs, ys, zs, hs;
     DevBuf packed, shadowHi, shadowLo; // x,y,z,h records of the keys pass; float shadows made by the gather
-    DevBuf pout;                       // per particle: outside its leaf's box (neighbour search)
+    DevBuf pnode;                      // per particle: its leaf's node, and whether it lies outside the leaf's box
     DevBuf sortWs, errWords;
     DevBuf buildWs, leaves, counts, layout;
     DevBuf prefixes, childOffsets, parents, levelRange, i2l, l2i, linkWs;
@@ -296,7 +296,7 @@ struct Pipeline final : PipelineBase
         if (cfg.do_neighbors)
         {
             if ((rc = nb.ensure(std::max<size_t>(1, nIn * cfg.ngmax) * sizeof(uint32_t)))) return rc;
-            if ((rc = pout.ensure(nIn))) return rc;
+            if ((rc = pnode.ensure(nIn * sizeof(uint32_t)))) return rc;
         }
         return CS_OK;
     }
@@ -371,9 +371,9 @@ struct Pipeline final : PipelineBase
                 return rc;
             if ((rc = nbMarkOutside<T>(s, xs.as<T>(), ys.as<T>(), zs.as<T>(), prep.phi, centers.as<T>(),
                                        sizes.as<T>(), childOffsets.as<int32_t>(), i2l.as<int32_t>(),
-                                       layout.as<uint32_t>(), Ncap, prep, pout.as<uint8_t>(), Ldev)))
+                                       layout.as<uint32_t>(), Ncap, prep, pnode.as<uint32_t>(), Ldev)))
                 return rc;
-            prep.pout = pout.as<uint8_t>();
+            prep.pnode = pnode.as<uint32_t>();
         }
         CSG_CUDA_TRY(rec(ev[ST_HALOS]));
         CSG_CUDA_TRY(rec(ev[ST_NEIGHBORS]));
@@ -384,8 +384,7 @@ struct Pipeline final : PipelineBase
             NbArgs<T> a = makeNbArgs<T>(xs.as<T>(), ys.as<T>(), zs.as<T>(), hs.as<T>(), 0, uint32_t(nIn), box, nv,
                                         cfg.ngmax, nb.as<uint32_t>(), nc.as<uint32_t>());
             a.errWord   = err + 3;
-            a.groupSize    = tuning.nb_group;
-            a.byTargetCost = tuning.nb_by_target_cost;
+            a.groupSize = tuning.nb_group;
             if ((rc = findNeighbors<T>(s, a, prep))) return rc;
         }
         CSG_CUDA_TRY(rec(ev[ST_COUNT]));
@@ -518,7 +517,7 @@ struct Pipeline final : PipelineBase
         size_t t = 0;
         for (const DevBuf* b : {&inBuf[0][0], &inBuf[0][1], &inBuf[0][2], &inBuf[0][3], &inBuf[1][0], &inBuf[1][1],
                                 &inBuf[1][2], &inBuf[1][3], &keys, &keysAlt, &order, &orderAlt, &xs, &ys, &zs, &hs,
-                                &packed, &shadowHi, &shadowLo, &pout, &sortWs, &errWords, &buildWs, &leaves, &counts,
+                                &packed, &shadowHi, &shadowLo, &pnode, &sortWs, &errWords, &buildWs, &leaves, &counts,
                                 &layout, &prefixes, &childOffsets, &haloList,
                                 &parents, &levelRange, &i2l, &l2i, &linkWs, &centers, &sizes, &sc, &ss, &flags,
                                 &nbPrepWs, &nb, &nc, &ncAlt, &flagsAlt})
@@ -712,12 +711,12 @@ struct Pipeline final : PipelineBase
         {
             const size_t nbNeed = std::max<size_t>(1, n * cfg.ngmax) * sizeof(uint32_t);
             if ((rc = nb.ensure(nbNeed))) return rc;
-            if ((rc = pout.ensure(n))) return rc;
+            if ((rc = pnode.ensure(n * sizeof(uint32_t)))) return rc;
             if ((rc = nbMarkOutside<T>(s, xs.as<T>(), ys.as<T>(), zs.as<T>(), prep.phi, centers.as<T>(),
                                        sizes.as<T>(), childOffsets.as<int32_t>(), i2l.as<int32_t>(),
-                                       layout.as<uint32_t>(), N, prep, pout.as<uint8_t>())))
+                                       layout.as<uint32_t>(), N, prep, pnode.as<uint32_t>())))
                 return rc;
-            prep.pout = pout.as<uint8_t>();
+            prep.pnode = pnode.as<uint32_t>();
         }
 
         // ---- halos for the focus leaves ----
@@ -753,8 +752,7 @@ struct Pipeline final : PipelineBase
             NbArgs<T> a = makeNbArgs<T>(xs.as<T>(), ys.as<T>(), zs.as<T>(), hs.as<T>(), 0, uint32_t(n), box, nv,
                                         cfg.ngmax, nb.as<uint32_t>(), nc.as<uint32_t>());
             a.errWord   = err + 3;
-            a.groupSize    = tuning.nb_group;
-            a.byTargetCost = tuning.nb_by_target_cost;
+            a.groupSize = tuning.nb_group;
             if (statsOn)
             {
                 if ((rc = nbStats.ensure(32 * sizeof(unsigned long long)))) return rc;
@@ -767,39 +765,13 @@ struct Pipeline final : PipelineBase
                 unsigned long long h[32];
                 CSG_CUDA_TRY(cudaMemcpyAsync(h, nbStats.p, sizeof(h), cudaMemcpyDeviceToHost, s));
                 CSG_CUDA_TRY(cudaStreamSynchronize(s));
+                const double wn = double(std::max(1ull, h[7]));
                 std::fprintf(stderr,
-                             "[cstone_gb300 neighbour stats] warps %llu | per warp: node expansions %.1f leaves %.1f "
-                             "candidates %.1f | lane cell tests %llu (fp64 %llu) | lane pair tests %llu "
-                             "(exact %llu)\n",
-                             h[7], double(h[6]) / h[7], double(h[4]) / h[7], double(h[5]) / h[7], h[0], h[1], h[2],
+                             "[cstone_gb300 neighbour stats] warps %llu | per warp: node expansions %.1f in %.1f steps, leaves %.1f "
+                             "candidates read %.1f in %.1f rounds, kept %.1f in %.1f tiles, rounds target by target %.2f "
+                             "| FP32 re-tests %llu exact decisions %llu\n",
+                             h[7], h[6] / wn, h[12] / wn, h[4] / wn, h[5] / wn, h[10] / wn, h[8] / wn, h[9] / wn, h[11] / wn, h[2],
                              h[3]);
-                std::fprintf(stderr,
-                             "[cstone_gb300 neighbour stats] slowest warp: %llu cycles, expansions %llu leaves %llu "
-                             "candidates %llu loose %llu first target %llu | loose warps %llu\n",
-                             h[8], h[9], h[10], h[11], h[12], h[13], h[14]);
-                auto asf = [](unsigned long long v) {
-                    unsigned u = unsigned(v);
-                    float f;
-                    std::memcpy(&f, &u, 4);
-                    return double(f);
-                };
-                std::fprintf(stderr,
-                             "[cstone_gb300 neighbour stats] slowest warp geometry: rmax %g rmin %g group radius %g "
-                             "box half %g C %g\n",
-                             asf(h[15]), asf(h[18]), asf(h[16]), asf(h[17]), asf(h[19]));
-                std::fprintf(stderr,
-                             "[cstone_gb300 neighbour stats] candidate batches %.1f per warp, steps %.1f, needing "
-                             "lanes %.1f, min-cost/step-cost %.3f | cycles in batches %.1f%% of warp cycles\n",
-                             double(h[23]) / h[7], double(h[20]) / h[23], double(h[21]) / h[23],
-                             double(h[22]) / (11.0 * double(h[20])), 100.0 * double(h[24]) / double(h[25]));
-                std::fprintf(stderr,
-                             "[cstone_gb300 neighbour stats] cycles in leaf visits %.1f%% | leaf visits no lane "
-                             "needed %.1f per warp\n",
-                             100.0 * double(h[26]) / double(h[25]), double(h[27]) / h[7]);
-                std::fprintf(stderr,
-                             "[cstone_gb300 neighbour stats] output per warp: sum of the most hits of a lane per "
-                             "batch %.1f, lanes with hits %.1f, rounds of 32 hits %.1f | exact path walks %.2f\n",
-                             double(h[28]) / h[7], double(h[29]) / h[7], double(h[30]) / h[7], double(h[31]) / h[7]);
             }
         }
         CSG_CUDA_TRY(cudaEventRecord(ev[ST_COUNT], s));

@@ -583,10 +583,9 @@ int cs_pipeline_reset_steps(cs_pipeline p);
 int cs_pipeline_graph_replays(cs_pipeline p);
 
 /* ---- tuning: knobs that change the speed of a pipeline, never its results -----------------------------------------
- * nb_group: targets per warp of the neighbour traversal (32, 16 or 8; 1, 2 or 4 lanes per target).
- * nb_by_target_cost: with one target per lane, a candidate batch that few lanes need runs the by-target loop (lanes
- * hold the candidates, the warp loops over the needing targets) when 19 x (needing lanes) < nb_by_target_cost x (the
- * per-lane loop's candidate steps); 0 never.
+ * nb_group: targets per warp of the neighbour traversal (32: pair tests on tensor-core tiles; 16 or 8: 2 or 4 lanes
+ * per target).
+ * nb_by_target_cost: accepted and kept for callers that set it; no kernel depends on it any more.
  * sort_items: the key sort's tile shape, keys per thread (16 with 3 blocks of 256 threads per SM, or 12 with 4; 0
  * means 16). Default {32, 7, 16}. Setting a tuning ends a step sequence (the next cs_pipeline_step builds from the
  * root). The reference has no counterpart: its traversal shape is the compile-time TravConfig

@@ -1,0 +1,88 @@
+"""GPU parity of the tiled neighbour search (32 targets x 32 candidates per tensor-core tile) at the places where it can
+go wrong: sets that end inside a warp or a tile, rows that fill up inside a tile, targets too spread or with radii too
+different for a tile, particles at one point or exactly at the radius, sets far from the origin, coarse keys (most
+particles outside their leaf's box) and cell radii below and above the search radius. Counts and lists equal the oracle's
+exactly; the smaller groups of the tuning take the other kernel and must agree too."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import neighbor_lists_equal, to_dev, u32, uniform
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(cs, O, x, y, z, h, bucket, ngmax, kind=1, bits=64, ext=1.0, lo=None, hi=None):
+    lo = lo if lo is not None else [float(a.min()) - 1e-3 for a in (x, y, z)]
+    hi = hi if hi is not None else [float(a.max()) + 1e-3 for a in (x, y, z)]
+    ref = O.pipeline(x, y, z, h, O.make_box(lo, hi), bucket, ngmax, kind, bits, ext)
+    p = cs.Pipeline(64 if x.dtype == np.float64 else 32, bits, kind, bucket, ngmax, ext, 1.0, False, True)
+    t = to_dev(x, y, z, h)
+    for group in (32, 16):
+        p.set_tuning(group, 7)
+        p.run(*t, cs.make_box(lo, hi))
+        out = p.outputs()
+        torch.cuda.synchronize()
+        neighbor_lists_equal(u32(out["neighbors"]).reshape(-1, ngmax), u32(out["neighbor_counts"]), ref["nb"], ref["nc"],
+                             ngmax)
+    return ref["nc"]
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 65, 96, 97, 500, 4100])
+def test_sizes_around_warps_and_tiles(cs, O, n, dtype):
+    x, y, z = uniform(O, 100 + n, n, -1.0, 1.0, dtype)
+    h = np.full(n, 0.5 * (3 * 40 * 8 / (4 * np.pi * max(n, 60))) ** (1 / 3), dtype)
+    _check(cs, O, x, y, z, h, 8, 64)
+
+
+@pytest.mark.parametrize("ngmax", [1, 7, 32, 33])
+def test_rows_that_fill_up(cs, O, ngmax):
+    x, y, z = uniform(O, 5, 1500, -1.0, 1.0)
+    nc = _check(cs, O, x, y, z, np.full(1500, 0.25), 16, ngmax)
+    assert nc.max() > ngmax
+    assert _check(cs, O, x, y, z, np.full(1500, 4.0), 16, ngmax).min() == 1499  # everything is a neighbour
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_radii_and_spreads_beyond_a_tile(cs, O, dtype):
+    rng = np.random.default_rng(3)
+    n = 6000
+    x, y, z = uniform(O, 7, n, -1.0, 1.0, dtype)
+    h = (0.05 * 10.0 ** rng.uniform(-2.5, 0.5, n)).astype(dtype)
+    h[::97] = 0.0
+    _check(cs, O, x, y, z, h, 16, 100)
+    # clumps far apart along a Morton curve, radii of the clumps' size
+    c = rng.integers(0, 40, n)
+    centres = rng.uniform(-50.0, 50.0, (3, 40))
+    x, y, z = ((centres[k][c] + rng.normal(0, 0.01, n)).astype(dtype) for k in range(3))
+    _check(cs, O, x, y, z, np.full(n, 0.004, dtype), 16, 100, kind=0)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_coincident_particles_and_pairs_at_the_radius(cs, O, dtype):
+    rng = np.random.default_rng(4)
+    pts = rng.uniform(-1.0, 1.0, (5, 3))
+    x, y, z = (pts[rng.integers(0, 5, 700)][:, k].astype(dtype) for k in range(3))
+    _check(cs, O, x, y, z, np.full(700, 1e-3, dtype), 64, 200)
+    # a lattice whose spacing is the radius, and one whose face diagonal nearly is (strict <)
+    g = np.arange(16) / 8.0
+    x, y, z = (a.reshape(-1).astype(dtype) for a in np.meshgrid(g, g, g, indexing="ij"))
+    for r in (0.125, np.nextafter(dtype(0.125), dtype(1)), 0.125 * np.sqrt(2.0), 0.25):
+        _check(cs, O, x, y, z, np.full(x.size, dtype(r) / dtype(2), dtype), 16, 64, lo=(0, 0, 0), hi=(2, 2, 2))
+
+
+@pytest.mark.parametrize("offset", [1e3, 1e6, -3e8])
+def test_sets_far_from_the_origin(cs, O, offset):
+    x, y, z = uniform(O, 9, 3000, 0.0, 1.0)
+    h = np.full(3000, 0.06)
+    _check(cs, O, x + offset, y - offset, z + 2 * offset, h, 16, 100)
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("ext", [0.8, 1.0, 1.3])
+def test_coarse_keys_and_cell_radii(cs, O, kind, ext):
+    n = 30000
+    x, y, z = (a.astype(np.float32) for a in O.plummer(31, n))
+    lo, hi = [float(a.min()) for a in (x, y, z)], [float(a.max()) for a in (x, y, z)]
+    _check(cs, O, x, y, z, np.full(n, 0.06, np.float32), 16, 100, kind, 32, ext, lo, hi)
