@@ -5,10 +5,10 @@
 // Search boxes: 8 lanes per leaf stride over its particles; min/max are exact (taken on order-preserving integer
 // images of the values), so any reduction order gives the reference's bits (up to the sign of a zero extremum that
 // ties with the other zero). FP64 particles go through an FP32 screen first, and only the particles that can hold an
-// extremum are evaluated in FP64 (searchBoxesScreenKernel). Collisions: the containment test per focus leaf, then one
-// warp-wide traversal testing 32 nodes at a time for each leaf that needs it, either in the warp that owns 32
-// neighbouring leaves (findHalosWarpKernel) or, given a scratch list, by persistent warps over the list of leaves
-// that need one (haloNeedKernel, findHalosListKernel); the flagged set equals that of the reference's per-leaf
+// extremum are evaluated in FP64 (searchBoxesScreenKernel). Collisions: the containment test per focus leaf, then a
+// traversal for each leaf that needs it: by persistent warps over the list of those leaves, long traversals handed on in
+// pieces (haloNeedKernel, findHalosListKernel), or, without scratch memory, by the warp that owns 32 neighbouring leaves
+// (findHalosWarpKernel); the flagged set equals that of the reference's per-leaf
 // singleTraversal (traversal/traversal.hpp:26-69), and every floating-point expression is unfused and in the
 // reference's order.
 #include "cs_common.cuh"
@@ -635,15 +635,42 @@ __global__ void __launch_bounds__(32 * HALO_WARPS)
     }
 }
 
-// With a scratch list the work is split in two launches, so that the traversals spread over the whole GPU instead of
-// running one after another in the warp that owns 32 neighbouring leaves (the leaves near the focus boundary are
-// few and clustered). haloNeedKernel: one thread per focus leaf decides the containment test and appends the leaves
-// that need a traversal (warp-aggregated; the order of the list does not matter, since the flagged set does not
-// depend on the visiting order). findHalosListKernel: persistent warps take list entries one at a time from a
-// counter and traverse for each. scratch: [0] list length, [1] next entry, [2 ...] the list.
+// With scratch memory the work is split, so that the traversals spread over the whole GPU instead of running one after
+// another in the warp that owns 32 neighbouring leaves (the leaves near the focus boundary are few and clustered).
+// haloNeedKernel: one thread per focus leaf decides the containment test and appends the leaves that need a traversal
+// (warp-aggregated; the order of the list does not matter, since the flagged set does not depend on the visiting order).
+// findHalosListKernel, HALO_PASSES launches: persistent warps take list entries one at a time from a counter and traverse
+// for each. A traversal can be as long as the tree (one leaf of a Plummer sphere's outskirts has a search box that holds
+// the core), so an entry that is not done after some steps appends what it has left to the next pass's list, one entry
+// per sibling group, and the pieces spread again. Breadth first in those steps: a tree's nodes concentrate in one or two
+// children per level (the core), and a frontier of 16 steps divides them where the stack of a depth-first walk keeps
+// them together. 51 such leaves of a 120k-particle set walk 83 thousand nodes; on 51 of the GPU's 24 thousand groups
+// that took 1.3 ms, handed on twice depth first 0.47 ms, handed on four times breadth first 0.1 ms.
+constexpr int HALO_PASSES = 5;
+constexpr int HALO_MORE   = 1 << 17; // entries of a later pass's list
+
+struct HaloScratch
+{
+    int32_t* base; // [2 p]: length of pass p's list, [2 p + 1]: its next entry
+    int32_t* need; // pass 0: leaves
+    int2* more[2]; // pass p: more[p & 1], (leaf, first node of a sibling group)
+};
+
+static HaloScratch haloScratch(int32_t* scratch, size_t numFocus)
+{
+    HaloScratch h;
+    h.base    = scratch;
+    h.need    = scratch + 16;
+    h.more[0] = reinterpret_cast<int2*>(h.need + ((numFocus + 1) & ~size_t(1)));
+    h.more[1] = h.more[0] + HALO_MORE;
+    return h;
+}
+
+size_t haloScratchInts(size_t numFocus) { return 16 + ((numFocus + 1) & ~size_t(1)) + 4 * size_t(HALO_MORE); }
+
 template<class K, class T>
 __global__ void haloNeedKernel(const K* __restrict__ leaves, const T* __restrict__ sc, const T* __restrict__ ss,
-                               BoxParams<T> b, KeyParams<T, K> kp, int firstNode, int lastNode, int32_t* scratch)
+                               BoxParams<T> b, KeyParams<T, K> kp, int firstNode, int lastNode, HaloScratch scratch)
 {
     const long long leaf = firstNode + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     bool need            = false;
@@ -662,16 +689,19 @@ __global__ void haloNeedKernel(const K* __restrict__ leaves, const T* __restrict
     if (m == 0) return;
     const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
     int base       = 0;
-    if (lane == leader) base = atomicAdd(&scratch[0], __popc(m));
+    if (lane == leader) base = atomicAdd(&scratch.base[0], __popc(m));
     base = __shfl_sync(0xffffffffu, base, leader);
-    if (need) scratch[2 + base + __popc(m & ((1u << lane) - 1u))] = int32_t(leaf);
+    if (need) scratch.need[base + __popc(m & ((1u << lane) - 1u))] = int32_t(leaf);
 }
 
-// Per 8-lane group: its own traversal of one list entry at a time, one sibling group of 8 nodes per step from its
+// findHalosListKernel. Per 8-lane group: its own traversal of one list entry at a time, one sibling group of 8 nodes per step from its
 // own LIFO stack, so that a warp keeps four traversals in flight (a traversal's stack is mostly shallow, and each
-// step waits for its node loads). One group popped and at most 8 pushed per step bounds a stack by 7 entries per
-// level plus 8 (7 * 21 + 8 = 155 for 64-bit keys).
-constexpr int HALO_GSTACK = 160;
+// step waits for its node loads). Depth first, one group popped and at most 8 pushed per step bound the stack by 7
+// entries per level plus 8 (7 * 21 + 8 = 155 for 64-bit keys); the HALO_BREADTH breadth-first steps before it leave at
+// most 1 + 7 * 16 = 113 entries (and use 1 + 8 * 16 places).
+constexpr int HALO_BREADTH = 16;
+constexpr int HALO_DEPTH   = 64;
+constexpr int HALO_GSTACK = 272;
 
 template<class K, class T, bool FloatFilter>
 __global__ void __launch_bounds__(32 * HALO_WARPS, 10)
@@ -679,33 +709,48 @@ __global__ void __launch_bounds__(32 * HALO_WARPS, 10)
                         const T* __restrict__ nc, const T* __restrict__ ns, const K* __restrict__ leaves,
                         const T* __restrict__ sc, const T* __restrict__ ss, BoxParams<T> b, int firstNode,
                         int lastNode, uint8_t* flags, uint32_t* errWord, const float4* __restrict__ nrec,
-                        int32_t* scratch)
+                        HaloScratch scratch, int pass)
 {
     __shared__ int sStack[HALO_WARPS][4][HALO_GSTACK];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 3, sub = lane & 7, lead = lane & ~7;
-    const int total = scratch[0];
+    int total = scratch.base[2 * pass];
+    if (pass > 0) total = min(total, HALO_MORE);
     if (total == 0) return;
-    const K lowest  = leaves[firstNode];
-    const K highest = leaves[lastNode];
-    int* stack      = sStack[warp][g];
-    int top         = 0;     // the group's stack height (the same in its 8 lanes)
-    bool done       = false; // the group found the list exhausted
+    // steps after which an entry hands the rest on: with fewer entries than groups early, so that the idle groups get
+    // work; otherwise only where one entry would outlast the others. A step is one round trip to L2 (0.6 us)
+    const bool few   = pass < HALO_PASSES - 1 && total < int(gridDim.x) * HALO_WARPS * 4;
+    const int budget = pass == HALO_PASSES - 1 ? INT_MAX : (few ? HALO_BREADTH : HALO_DEPTH);
+    const K lowest   = leaves[firstNode];
+    const K highest  = leaves[lastNode];
+    int* stack       = sStack[warp][g];
+    int low = 0, top = 0;     // the group's entries: stack[low] .. stack[top - 1] (the same in its 8 lanes)
+    bool done        = false; // the group found the list exhausted
+    int leaf         = 0;
+    int steps        = 0;
     T tc[3] = {}, ts[3] = {};
     float tcf[3] = {}, tsf[3] = {};
     for (;;)
     {
-        // a group without work takes the next list entry; its lane 0 tests the root
-        const bool want = !done && top == 0;
+        // a group without work takes the next list entry; a leaf's traversal begins with its lane 0 testing the root
+        const bool want = !done && top == low;
         int item        = 0;
-        if (want && sub == 0) item = atomicAdd(&scratch[1], 1);
+        if (want && sub == 0) item = atomicAdd(&scratch.base[2 * pass + 1], 1);
         item = __shfl_sync(0xffffffffu, item, lead);
+        int start = 0;
         if (want)
         {
             if (item >= total)
                 done = true;
             else
             {
-                const int leaf = scratch[2 + item];
+                if (pass == 0) { leaf = scratch.need[item]; }
+                else
+                {
+                    const int2 m = scratch.more[pass & 1][item];
+                    leaf         = m.x;
+                    start        = m.y;
+                }
+                steps = low = top = 0;
 #pragma unroll
                 for (int k = 0; k < 3; ++k)
                 {
@@ -717,20 +762,19 @@ __global__ void __launch_bounds__(32 * HALO_WARPS, 10)
             }
         }
         if (__all_sync(0xffffffffu, done)) return;
-        int rootChild = 0;
-        if (want && !done && sub == 0)
+        if (pass == 0 && want && !done && sub == 0)
         {
             float4 c4{}, s4{};
             haloRecords<T, FloatFilter>(nrec, 0, c4, s4);
             const int ch = childOffsets[0];
             if (haloNodeTest<K, T, FloatFilter>(0, prefixes[0], c4, s4, tc, ts, tcf, tsf, lowest, highest, nc, ns, b,
                                                 flags))
-                rootChild = ch;
+                start = ch;
         }
-        rootChild = __shfl_sync(0xffffffffu, rootChild, lead);
-        if (rootChild != 0)
+        start = __shfl_sync(0xffffffffu, start, lead);
+        if (start != 0)
         {
-            if (sub == 0) stack[0] = rootChild;
+            if (sub == 0) stack[0] = start;
             top = 1;
         }
         __syncwarp();
@@ -739,10 +783,11 @@ __global__ void __launch_bounds__(32 * HALO_WARPS, 10)
         // groups of the overlapping internal ones
         bool push = false;
         int child = 0;
-        if (top > 0)
+        if (top > low)
         {
-            --top;
-            const int node = stack[top] + sub;
+            const int at = few && steps < HALO_BREADTH ? low++ : --top;
+            ++steps;
+            const int node = stack[at] + sub;
             const K pfx    = prefixes[node];
             const int ch   = childOffsets[node];
             float4 c4{}, s4{};
@@ -764,6 +809,33 @@ __global__ void __launch_bounds__(32 * HALO_WARPS, 10)
         if (push) stack[top + __popc(pm & ((1u << sub) - 1u))] = child;
         top += __popc(pm);
         __syncwarp();
+
+        // out of steps: the rest goes to the next pass as far as its list has room, and is walked here beyond that
+        const bool hand = top > low && steps == budget;
+        if (__any_sync(0xffffffffu, hand))
+        {
+            int at = 0;
+            if (hand && sub == 0) at = atomicAdd(&scratch.base[2 * pass + 2], top - low);
+            at = __shfl_sync(0xffffffffu, at, lead);
+            if (hand)
+            {
+                const int room = max(0, min(top - low, HALO_MORE - at));
+                top -= room;
+                for (int k = sub; k < room; k += 8)
+                    scratch.more[(pass + 1) & 1][at + k] = make_int2(leaf, stack[top + k]);
+                // what stays moves to the stack's bottom, eight entries at a time
+                for (int k = 0; k < top - low; k += 8)
+                {
+                    const int e = low + k + sub < top ? stack[low + k + sub] : 0;
+                    __syncwarp(0xffu << lead);
+                    if (low + k + sub < top) stack[k + sub] = e;
+                    __syncwarp(0xffu << lead);
+                }
+                top -= low;
+                low = 0;
+            }
+            __syncwarp();
+        }
     }
 }
 
@@ -793,26 +865,36 @@ int findHalos(cudaStream_t s, const K* prefixes, const int32_t* childOffsets, co
     bool anyPbc = bp.pbc[0] || bp.pbc[1] || bp.pbc[2];
     bool ff     = false;
     if constexpr (std::is_same_v<T, double>) ff = nrec && !anyPbc;
+    Workspace own;
+    if (!scratch)
+    {
+        // a caller without scratch memory: taken from the stream's pool, unless the stream is being captured or the
+        // memory is not there
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+            own.acquire(nullptr, 0, haloScratchInts(size_t(last - first)) * sizeof(int32_t), s) == CS_OK)
+            scratch = static_cast<int32_t*>(own.ptr);
+        else
+            (void)cudaGetLastError();
+    }
     if (scratch)
     {
-        CSG_CUDA_TRY(cudaMemsetAsync(scratch, 0, 2 * sizeof(int32_t), s));
-        haloNeedKernel<K, T><<<iceil(size_t(last - first), 256), 256, 0, s>>>(leaves, sc, ss, bp, kp, first, last,
-                                                                             scratch);
+        const HaloScratch hs = haloScratch(scratch, size_t(last - first));
+        CSG_CUDA_TRY(cudaMemsetAsync(hs.base, 0, 16 * sizeof(int32_t), s));
+        haloNeedKernel<K, T><<<iceil(size_t(last - first), 256), 256, 0, s>>>(leaves, sc, ss, bp, kp, first, last, hs);
         CSG_CHECK_LAUNCH();
-        if constexpr (std::is_same_v<T, double>)
-        {
-            if (ff)
+        auto passes = [&](auto kernel, int grid, const float4* records) -> int {
+            for (int pass = 0; pass < HALO_PASSES; ++pass)
             {
-                findHalosListKernel<K, T, true><<<haloListGrid<K, T, true>(), 32 * HALO_WARPS, 0, s>>>(
-                    prefixes, childOffsets, nc, ns, leaves, sc, ss, bp, first, last, flags, errWord, nrec, scratch);
+                kernel<<<grid, 32 * HALO_WARPS, 0, s>>>(prefixes, childOffsets, nc, ns, leaves, sc, ss, bp, first, last,
+                                                        flags, errWord, records, hs, pass);
                 CSG_CHECK_LAUNCH();
-                return CS_OK;
             }
-        }
-        findHalosListKernel<K, T, false><<<haloListGrid<K, T, false>(), 32 * HALO_WARPS, 0, s>>>(
-            prefixes, childOffsets, nc, ns, leaves, sc, ss, bp, first, last, flags, errWord, nullptr, scratch);
-        CSG_CHECK_LAUNCH();
-        return CS_OK;
+            return CS_OK;
+        };
+        if constexpr (std::is_same_v<T, double>)
+            if (ff) return passes(findHalosListKernel<K, T, true>, haloListGrid<K, T, true>(), nrec);
+        return passes(findHalosListKernel<K, T, false>, haloListGrid<K, T, false>(), nullptr);
     }
     unsigned blocks = iceil(size_t(last - first), 32 * HALO_WARPS);
     if constexpr (std::is_same_v<T, double>)

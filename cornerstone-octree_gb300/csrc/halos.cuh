@@ -15,11 +15,13 @@ int searchBoxes(cudaStream_t s, const T* x, const T* y, const T* z, const Th* h,
 
 //! nrec (may be null): the neighbour search's float node records (NbPrep::nrec: centre and half size rounded to
 //! nearest at [3i] and [3i + 2]); with T = double and no periodic axis they enable the float pre-filter of the node
-//! test. scratch (may be null): (last - first + 2) int32 of device memory for the list of leaves that need a
-//! traversal; with it the traversals run on persistent warps over that list
+//! test. scratch (may be null: taken from the stream's pool, or done without while the stream is being captured):
+//! haloScratchInts(last - first) int32 of device memory, 8-byte aligned, for the lists of what is left to traverse
 template<class K, class T>
 int findHalos(cudaStream_t s, const K* prefixes, const int32_t* childOffsets, const int32_t* parents, const T* nc,
               const T* ns, const K* leaves, const T* sc, const T* ss, const cs_box& box, int first, int last,
               uint8_t* flags, uint32_t* errWord, const float4* nrec, int32_t* scratch = nullptr);
+
+size_t haloScratchInts(size_t numFocus);
 
 } // namespace csg

@@ -735,7 +735,8 @@ struct Pipeline final : PipelineBase
                 return rc;
             if constexpr (!(std::is_same_v<K, uint32_t> && std::is_same_v<T, double>))
             {
-                if ((rc = haloList.ensure((size_t(br.focusLast - br.focusFirst) + 2) * sizeof(int32_t)))) return rc;
+                if ((rc = haloList.ensure(haloScratchInts(size_t(br.focusLast - br.focusFirst)) * sizeof(int32_t))))
+                    return rc;
                 if ((rc = findHalos<K, T>(s, prefixes.as<K>(), childOffsets.as<int32_t>(), parents.as<int32_t>(),
                                           centers.as<T>(), sizes.as<T>(), leaves.as<K>(), sc.as<T>(), ss.as<T>(), box,
                                           br.focusFirst, br.focusLast, flags.as<uint8_t>(), err + 2, prep.nrec,
