@@ -11,6 +11,10 @@
 // Entries past list_capacity are not written; offsets[n] always holds the total, so the caller can tell. The
 // pipeline's host-buffer runs compact into device memory and copy the list to the host with the copy engine.
 //
+// A tile is one row per thread, so that a warp copies only 32 rows one after another (four rows' loads in flight): tiles
+// of 2048 rows left 244 blocks for 500k rows and a serial chain of 256 rows per warp, 0.54 ms for 200 MB of list where
+// this form takes 0.13 ms; 16M rows of 100 entries: 4.6 -> 3.7 ms.
+//
 // Algorithmic bytes: reads 4 n (counts) + 4 total (stored entries), writes 8 (n + 1) + 4 total.
 #include "cs_common.cuh"
 #include "neighbor_csr.cuh"
@@ -19,8 +23,8 @@ namespace csg
 {
 
 constexpr int CSR_THREADS = 256;
-constexpr int CSR_ROWS    = 8;                          // rows per thread in the scans
-constexpr int CSR_TILE    = CSR_THREADS * CSR_ROWS;     // rows per block
+constexpr int CSR_TILE    = CSR_THREADS; // rows per block
+constexpr int CSR_SUMS    = 8;           // tile sums per thread and round of their scan
 
 __device__ __forceinline__ unsigned long long blockExclusiveScanU64(unsigned long long v, unsigned long long* sWarp,
                                                                     unsigned long long* total)
@@ -58,11 +62,8 @@ __global__ void __launch_bounds__(CSR_THREADS) csrTileSumsKernel(const uint32_t*
                                                                   unsigned ngmax, unsigned long long* tileSums)
 {
     __shared__ unsigned long long sWarp[CSR_THREADS / 32];
-    size_t base = size_t(blockIdx.x) * CSR_TILE + size_t(threadIdx.x) * CSR_ROWS;
-    unsigned long long v = 0;
-#pragma unroll
-    for (int k = 0; k < CSR_ROWS; ++k)
-        if (base + k < n) v += min(__ldg(nc + base + k), ngmax);
+    const size_t i             = size_t(blockIdx.x) * CSR_TILE + threadIdx.x;
+    const unsigned long long v = i < n ? min(__ldg(nc + i), ngmax) : 0u;
     unsigned long long total;
     blockExclusiveScanU64(v, sWarp, &total);
     if (threadIdx.x == 0) tileSums[blockIdx.x] = total;
@@ -76,13 +77,24 @@ __global__ void __launch_bounds__(CSR_THREADS) csrTileOffsetsKernel(unsigned lon
 {
     __shared__ unsigned long long sWarp[CSR_THREADS / 32];
     unsigned long long carry = 0;
-    for (int b = 0; b < numTiles; b += CSR_THREADS)
+    for (int b = 0; b < numTiles; b += CSR_THREADS * CSR_SUMS)
     {
-        int i                  = b + threadIdx.x;
-        unsigned long long v   = i < numTiles ? tileSums[i] : 0;
+        const int i0 = b + threadIdx.x * CSR_SUMS;
+        unsigned long long v[CSR_SUMS], sum = 0;
+#pragma unroll
+        for (int k = 0; k < CSR_SUMS; ++k)
+        {
+            v[k] = i0 + k < numTiles ? tileSums[i0 + k] : 0;
+            sum += v[k];
+        }
         unsigned long long total;
-        unsigned long long e = blockExclusiveScanU64(v, sWarp, &total);
-        if (i < numTiles) tileSums[i] = carry + e;
+        unsigned long long e = carry + blockExclusiveScanU64(sum, sWarp, &total);
+#pragma unroll
+        for (int k = 0; k < CSR_SUMS; ++k)
+        {
+            if (i0 + k < numTiles) tileSums[i0 + k] = e;
+            e += v[k];
+        }
         carry += total;
     }
     if (threadIdx.x == 0)
@@ -102,44 +114,34 @@ __global__ void __launch_bounds__(CSR_THREADS) csrWriteKernel(const uint32_t* __
     __shared__ unsigned long long sOff[CSR_TILE];
     __shared__ unsigned sCnt[CSR_TILE];
     const size_t tile0 = size_t(blockIdx.x) * CSR_TILE;
-    const int t0       = threadIdx.x * CSR_ROWS;
-    unsigned c[CSR_ROWS];
-    unsigned long long sum = 0;
-#pragma unroll
-    for (int k = 0; k < CSR_ROWS; ++k)
-    {
-        size_t i = tile0 + t0 + k;
-        c[k]     = i < n ? min(__ldg(nc + i), ngmax) : 0u;
-        sum += c[k];
-    }
+    const size_t i     = tile0 + threadIdx.x;
+    const unsigned c   = i < n ? min(__ldg(nc + i), ngmax) : 0u;
     unsigned long long total;
-    unsigned long long e = blockExclusiveScanU64(sum, sWarp, &total) + tileOffsets[blockIdx.x];
-#pragma unroll
-    for (int k = 0; k < CSR_ROWS; ++k)
-    {
-        sOff[t0 + k] = e;
-        sCnt[t0 + k] = c[k];
-        e += c[k];
-    }
-    __syncthreads();
-    // offsets: consecutive threads write consecutive rows
-    for (int r = threadIdx.x; r < CSR_TILE; r += CSR_THREADS)
-    {
-        size_t i = tile0 + r;
-        if (i < n) offsets[i] = sOff[r];
-    }
+    const unsigned long long e = blockExclusiveScanU64(c, sWarp, &total) + tileOffsets[blockIdx.x];
+    sOff[threadIdx.x]          = e;
+    sCnt[threadIdx.x]          = c;
+    if (i < n) offsets[i] = e;
     if (!list) return; // offsets only
-    // rows: warp w copies rows w, w + 8, ...; lanes copy 32 consecutive entries per round
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int r = warp; r < CSR_TILE; r += CSR_THREADS / 32)
+    __syncwarp();
+    // each warp its own 32 rows, four at a time; lanes copy 32 consecutive entries per round
+    constexpr int U = 4;
+    const int lane = threadIdx.x & 31, row0 = threadIdx.x & ~31;
+    for (int r = row0; r < row0 + 32; r += U)
     {
-        size_t i = tile0 + r;
-        if (i >= n) break;
-        const unsigned cnt           = sCnt[r];
-        const unsigned long long dst = sOff[r];
-        const uint32_t* src          = nb + i * size_t(ngmax);
-        for (unsigned k = lane; k < cnt; k += 32)
-            if (dst + k < capacity) list[dst + k] = __ldcs(src + k);
+        unsigned most = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            most = max(most, sCnt[r + u]);
+        for (unsigned k = lane; k < most; k += 32)
+        {
+            uint32_t v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                v[u] = k < sCnt[r + u] ? __ldcs(nb + (tile0 + r + u) * size_t(ngmax) + k) : 0u;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (k < sCnt[r + u] && sOff[r + u] + k < capacity) list[sOff[r + u] + k] = v[u];
+        }
     }
 }
 
