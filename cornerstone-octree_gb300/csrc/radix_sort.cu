@@ -2,9 +2,14 @@
 // "onesweep" kernel per 8-bit digit (Adinets & Merrill, "Onesweep: a faster least significant digit radix sort for
 // GPUs", 2022). Each block takes the next tile (256 threads x 16 or 12 keys: a runtime choice, SortShape) from an
 // atomic counter, ranks its keys by digit in input
-// order (warp match + per-warp counters), publishes its per-digit counts and obtains the counts of all earlier tiles
+// order (ballots + per-warp counters), publishes its per-digit counts and obtains the counts of all earlier tiles
 // by decoupled look-back, then scatters through shared memory so that global writes are runs of consecutive
 // addresses. Traffic per pass: 2 * (sizeof(K) + 4) bytes per pair; the histogram reads the keys once.
+//
+// What bounds it: latency and issue in equal parts (55 % of the issue slots at 24 warps per SM; a pass moves 2.0 to 2.3
+// TB/s, 30 to 35 % of the copy bandwidth). 16M 64-bit keys 1.68 -> 1.22 ms, 20M 32-bit keys 1.02 -> 0.70 ms with the
+// ballots in the ranking (a match instruction per key had bound every pass at 100 cycles each), pipelined counter
+// additions and four keys in flight per thread of the histogram (103 -> 52 us for 20M 32-bit keys).
 //
 // Look-back waits spin on a flag that an earlier tile (which has already started, because tiles are handed out in
 // order) will publish; every wait is bounded, and a wait that gives up sets ERRBIT_SORT_TIMEOUT and continues.
@@ -27,6 +32,11 @@ constexpr uint32_t ST_INC   = 2u << 30;
 constexpr uint32_t ST_FLAGS = 3u << 30;
 constexpr uint32_t ST_COUNT = (1u << 30) - 1;
 
+
+// resident blocks per SM of the 16-key tiles: what shared memory holds for 64-bit keys; 20M 32-bit keys 0.71 ms with 3,
+// 0.68 with 4, 0.93 with 5 (spilling)
+template<class K>
+constexpr int RS_BLOCKS16 = sizeof(K) == 4 ? 4 : 3;
 
 struct SortLayout
 {
@@ -77,26 +87,37 @@ __global__ void __launch_bounds__(256) radixHistogramKernel(const K* __restrict_
 
     const int copy = (threadIdx.x >> 5) & 1;
     const int lane = threadIdx.x & 31;
-    size_t stride  = size_t(gridDim.x) * blockDim.x;
-    for (size_t i0 = size_t(blockIdx.x) * blockDim.x; i0 < n; i0 += stride)
+    // four keys per thread and round, loaded before any is counted
+    constexpr int U     = 4;
+    const size_t stride = size_t(gridDim.x) * 256 * U;
+    for (size_t i0 = size_t(blockIdx.x) * 256 * U; i0 < n; i0 += stride)
     {
-        size_t i   = i0 + threadIdx.x;
-        bool valid = i < n;
-        K key      = valid ? keys[i] : K(0);
+        K key[U];
+        const bool full = i0 + 256 * U <= n;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+        {
+            const size_t i = i0 + u * 256 + threadIdx.x;
+            key[u]         = full || i < n ? keys[i] : K(0);
+        }
         for (int p = 0; p < passes; ++p)
         {
-            int shift     = beginBit + 8 * p;
-            int bitsHere  = min(8, endBit - shift);
-            uint32_t mask = (1u << bitsHere) - 1u;
-            uint32_t d    = digitOf(key, shift, mask);
-            uint32_t d0   = __shfl_sync(0xffffffffu, d, 0);
-            unsigned vmask = __ballot_sync(0xffffffffu, valid);
-            bool uniform   = __all_sync(0xffffffffu, !valid || d == d0) && (vmask & 1u);
-            if (uniform)
+            const int shift     = beginBit + 8 * p;
+            const uint32_t mask = (1u << min(8, endBit - shift)) - 1u;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
             {
-                if (lane == 0) atomicAdd(&sh[copy][p][d0], __popc(vmask));
+                const bool valid = full || i0 + u * 256 + threadIdx.x < n;
+                const uint32_t d = digitOf(key[u], shift, mask);
+                // one addition for a warp whose keys share the digit (the high digits of clustered or sorted keys)
+                int same;
+                __match_all_sync(0xffffffffu, valid ? d : ~0u, &same);
+                if (same)
+                {
+                    if (lane == 0 && valid) atomicAdd(&sh[copy][p][d], 32u);
+                }
+                else if (valid) { atomicAdd(&sh[copy][p][d], 1u); }
             }
-            else if (valid) { atomicAdd(&sh[copy][p][d], 1u); }
         }
     }
     __syncthreads();
@@ -134,6 +155,51 @@ __device__ __forceinline__ uint32_t blockExclusiveScan256(uint32_t v, uint32_t* 
     __syncthreads();
     uint32_t warpPrefix = warp > 0 ? sWarpSums[warp - 1] : 0;
     return warpPrefix + x - v;
+}
+
+// the lanes of the warp whose digit equals this lane's, by eight ballots: a match instruction takes time in proportion to
+// the distinct values (100 cycles of the shared-memory pipe for random digits)
+__device__ __forceinline__ unsigned digitPeers(uint32_t d)
+{
+    unsigned peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < 8; ++b)
+    {
+        const int set    = int(d << (31 - b)) >> 31; // all ones if bit b is set
+        const unsigned m = __ballot_sync(0xffffffffu, set != 0);
+        peers &= ~(m ^ unsigned(set));
+    }
+    return peers;
+}
+
+// rank of each of a warp's keys among the warp's keys of the same digit, in input order (item-major); hist (zero before)
+// then holds the warp's digit counts
+template<class K, int Items>
+__device__ __forceinline__ void rankItems(const K (&k)[Items], int shift, uint32_t mask, int lane, uint32_t* hist,
+                                          uint32_t (&rank)[Items])
+{
+    constexpr int Group   = 4; // items in flight
+    const unsigned ltMask = (1u << lane) - 1u;
+    static_assert(Items % Group == 0);
+#pragma unroll
+    for (int j0 = 0; j0 < Items; j0 += Group)
+    {
+        uint32_t old[Group];
+        unsigned peers[Group];
+#pragma unroll
+        for (int u = 0; u < Group; ++u)
+            peers[u] = digitPeers(digitOf(k[j0 + u], shift, mask));
+#pragma unroll
+        for (int u = 0; u < Group; ++u)
+        {
+            old[u] = 0;
+            if ((peers[u] >> lane) == 1u) old[u] = atomicAdd(hist + digitOf(k[j0 + u], shift, mask), __popc(peers[u]));
+            __syncwarp();
+        }
+#pragma unroll
+        for (int u = 0; u < Group; ++u)
+            rank[j0 + u] = __shfl_sync(0xffffffffu, old[u], 31 - __clz(peers[u])) + __popc(peers[u] & ltMask);
+    }
 }
 
 template<class K, bool Iota, int Items, int MinBlocks>
@@ -184,22 +250,10 @@ __global__ void __launch_bounds__(RS_THREADS, MinBlocks) onesweepKernel(const K*
         }
     }
 
-    // rank within the warp's 512-key sub-tile, in input order
+    // rank within the warp's sub-tile, in input order: the last lane of each digit's peers adds their number to the
+    // warp's counter and gets the count of earlier items back, several items in flight
     uint32_t rank[Items];
-    const unsigned ltMask = (1u << lane) - 1u;
-#pragma unroll
-    for (int j = 0; j < Items; ++j)
-    {
-        uint32_t d      = digitOf(k[j], shift, mask);
-        unsigned peers  = __match_any_sync(0xffffffffu, d);
-        int leader      = 31 - __clz(peers);
-        uint32_t before = __popc(peers & ltMask);
-        uint32_t base   = sWarpHist[warp][d];
-        __syncwarp();
-        if (lane == leader) sWarpHist[warp][d] = base + __popc(peers);
-        __syncwarp();
-        rank[j] = base + before;
-    }
+    rankItems<K, Items>(k, shift, mask, lane, sWarpHist[warp], rank);
     __syncthreads();
 
     // per digit (one thread per digit): tile total and per-warp exclusive prefixes
@@ -268,7 +322,7 @@ __global__ void __launch_bounds__(RS_THREADS, MinBlocks) onesweepKernel(const K*
         if (timedOut) atomicOr(errWord, ERRBIT_SORT_TIMEOUT);
         vstatus[myIdx] = ST_INC | (prefix + total);
     }
-    sGlobalBase[dg] = passHist[dg] + prefix;
+    sGlobalBase[dg] = passHist[dg] + prefix - excl; // global position of the tile's slot 0 were it of this digit
     __syncthreads();
 
     // scatter into shared memory in (digit, input order) order
@@ -288,13 +342,110 @@ __global__ void __launch_bounds__(RS_THREADS, MinBlocks) onesweepKernel(const K*
     {
         K key      = sKeys[i];
         uint32_t d = digitOf(key, shift, mask);
-        size_t out = size_t(sGlobalBase[d]) + (i - sTileOff[d]);
+        const uint32_t out = sGlobalBase[d] + uint32_t(i); // modulo 2^32, n < 2^30
         if (out < n)
         {
             keysOut[out] = key;
             valsOut[out] = sVals[i];
         }
     }
+}
+
+// Small sorts in one block: every pass in shared memory, 256 keys per warp, 8 per lane. The general path is ten dependent
+// launches of one or two tiles (4096 64-bit keys: 93 us of kernels, 27 us here), each a look-back, a histogram and a
+// trip through global memory; up to 8192 keys the block is faster, and its shared memory ends there.
+constexpr int SS_ITEMS = 8;
+constexpr int SS_MAX   = 32 * 32 * SS_ITEMS;
+
+template<class K>
+__global__ void __launch_bounds__(1024) smallSortKernel(K* keys, uint32_t* vals, int n, int beginBit, int endBit, int iota)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int slots = blockDim.x * SS_ITEMS, warps = blockDim.x >> 5;
+    K* sKeys        = reinterpret_cast<K*>(smem);
+    uint32_t* sVals = reinterpret_cast<uint32_t*>(sKeys + slots);
+    uint32_t* sHist = sVals + slots; // [warps][256]
+    __shared__ uint32_t sTileOff[RS_BINS];
+    __shared__ uint32_t sWarpSums[RS_WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, base = warp * 32 * SS_ITEMS;
+    K k[SS_ITEMS];
+    uint32_t v[SS_ITEMS];
+#pragma unroll
+    for (int j = 0; j < SS_ITEMS; ++j)
+    {
+        const int i = base + j * 32 + lane;
+        k[j]        = i < n ? keys[i] : ~K(0); // padding stays behind every key
+        v[j]        = i < n ? (iota ? uint32_t(i) : vals[i]) : 0u;
+    }
+    for (int shift = beginBit; shift < endBit; shift += 8)
+    {
+        const uint32_t mask = (1u << min(8, endBit - shift)) - 1u;
+        for (int b = tid; b < warps * RS_BINS; b += blockDim.x)
+            sHist[b] = 0;
+        __syncthreads();
+        uint32_t rank[SS_ITEMS];
+        rankItems<K, SS_ITEMS>(k, shift, mask, lane, sHist + warp * RS_BINS, rank);
+        __syncthreads();
+        uint32_t total = 0;
+        if (tid < RS_BINS)
+            for (int w = 0; w < warps; ++w)
+            {
+                const uint32_t c           = sHist[w * RS_BINS + tid];
+                sHist[w * RS_BINS + tid] = total;
+                total += c;
+            }
+        // exclusive scan of the 256 totals by the first eight warps
+        uint32_t x = total;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31 && warp < RS_WARPS) sWarpSums[warp] = x;
+        __syncthreads();
+        if (tid < RS_BINS)
+        {
+            uint32_t before = 0;
+            for (int w = 0; w < warp; ++w)
+                before += sWarpSums[w];
+            sTileOff[tid] = before + x - total;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < SS_ITEMS; ++j)
+        {
+            const uint32_t d   = digitOf(k[j], shift, mask);
+            const uint32_t pos = sTileOff[d] + sHist[warp * RS_BINS + d] + rank[j];
+            sKeys[pos]         = k[j];
+            sVals[pos]         = v[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < SS_ITEMS; ++j)
+        {
+            k[j] = sKeys[base + j * 32 + lane];
+            v[j] = sVals[base + j * 32 + lane];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < SS_ITEMS; ++j)
+    {
+        const int i = base + j * 32 + lane;
+        if (i < n) keys[i] = k[j], vals[i] = v[j];
+    }
+}
+
+template<class K>
+static int smallSort(cudaStream_t s, K* keys, uint32_t* vals, size_t n, int beginBit, int endBit, bool iota)
+{
+    const int warps    = std::max(RS_WARPS, int((n + 32 * SS_ITEMS - 1) / (32 * SS_ITEMS)));
+    const size_t bytes = size_t(warps) * (32 * SS_ITEMS * (sizeof(K) + sizeof(uint32_t)) + RS_BINS * sizeof(uint32_t));
+    CSG_CUDA_TRY(cudaFuncSetAttribute(smallSortKernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      int(32 * (32 * SS_ITEMS * (sizeof(K) + sizeof(uint32_t)) + RS_BINS * sizeof(uint32_t)))));
+    smallSortKernel<K><<<1, warps * 32, bytes, s>>>(keys, vals, int(n), beginBit, endBit, iota ? 1 : 0);
+    CSG_CHECK_LAUNCH();
+    return CS_OK;
 }
 
 __global__ void iotaKernel(uint32_t* v, size_t n)
@@ -397,13 +548,16 @@ int radixSortPairs(cudaStream_t s, K* keys, uint32_t* vals, K* keysAlt, uint32_t
         return CS_ERR_INVALID;
     }
     uint32_t* err = errWord;
+    // (the test mode that stalls a look-back needs one)
+    if (n <= size_t(SS_MAX) && !(waitLimits().stall & CS_WAIT_STALL_SORT))
+        return smallSort<K>(s, keys, vals, n, beginBit, endBit, iota);
 
     size_t zeroBytes = (reinterpret_cast<char*>(L.status + size_t(L.passes) * L.tiles * RS_BINS) -
                         reinterpret_cast<char*>(L.hist));
     CSG_CUDA_TRY(cudaMemsetAsync(L.hist, 0, zeroBytes, s));
 
     {
-        unsigned grid = unsigned(std::min<size_t>((n + 255) / 256, size_t(smCount()) * 8));
+        unsigned grid = unsigned(std::min<size_t>((n + 1023) / 1024, size_t(smCount()) * 8));
         radixHistogramKernel<K><<<grid, 256, 0, s>>>(keys, n, beginBit, endBit, passes, L.hist);
         CSG_CHECK_LAUNCH();
         histScanKernel<<<passes, RS_BINS, 0, s>>>(L.hist);
@@ -414,7 +568,7 @@ int radixSortPairs(cudaStream_t s, K* keys, uint32_t* vals, K* keysAlt, uint32_t
     uint32_t* vin = vals;
     int rc        = sortItems == 12
                         ? onesweepPasses<K, 12, 4>(s, kin, vin, keysAlt, valsAlt, n, beginBit, endBit, iota, L, err)
-                        : onesweepPasses<K, 16, 3>(s, kin, vin, keysAlt, valsAlt, n, beginBit, endBit, iota, L, err);
+                        : onesweepPasses<K, 16, RS_BLOCKS16<K>>(s, kin, vin, keysAlt, valsAlt, n, beginBit, endBit, iota, L, err);
     if (rc) return rc;
     bool inAlt = (kin == keysAlt);
     if (resultInAlt) { *resultInAlt = inAlt; }
@@ -433,8 +587,9 @@ int radixSortPreload()
     CSG_CUDA_TRY(cudaFuncGetAttributes(&fa, radixHistogramKernel<K>));
     CSG_CUDA_TRY(cudaFuncGetAttributes(&fa, histScanKernel));
     CSG_CUDA_TRY(cudaFuncGetAttributes(&fa, iotaKernel));
-    CSG_CUDA_TRY(cudaFuncGetAttributes(&fa, onesweepKernel<K, true, 16, 3>));
-    CSG_CUDA_TRY(cudaFuncGetAttributes(&fa, onesweepKernel<K, false, 16, 3>));
+    CSG_CUDA_TRY(cudaFuncGetAttributes(&fa, smallSortKernel<K>));
+    CSG_CUDA_TRY(cudaFuncGetAttributes(&fa, onesweepKernel<K, true, 16, RS_BLOCKS16<K>>));
+    CSG_CUDA_TRY(cudaFuncGetAttributes(&fa, onesweepKernel<K, false, 16, RS_BLOCKS16<K>>));
     CSG_CUDA_TRY(cudaFuncGetAttributes(&fa, onesweepKernel<K, true, 12, 4>));
     CSG_CUDA_TRY(cudaFuncGetAttributes(&fa, onesweepKernel<K, false, 12, 4>));
     return CS_OK;
