@@ -35,8 +35,9 @@
 // Only the tests that fall in [T_acc, T_out) are decided again in exact FP64, in out-of-line functions: inlined, the
 // compiler hoists their FP64 multiplies into the hot FP32 loop.
 //
-// Periodic boundaries. Warps that contain a target whose search sphere crosses a periodic boundary are served by the
-// per-lane path kernel (findNeighborsKernel): each lane keeps a mask per depth of its own root-to-node path and
+// Periodic boundaries. Warps that contain a target whose search sphere crosses a periodic boundary fold everything to the
+// image nearest to the targets (findNeighborsTileKernel's Fold instance), unless their spheres reach too far for one image:
+// those go to the per-lane path kernel (findNeighborsKernel): each lane keeps a mask per depth of its own root-to-node path and
 // decides every test in T exactly as the reference does, with minimum-image folding.
 #include "cs_common.cuh"
 #include "neighbors.cuh"
@@ -160,7 +161,31 @@ __device__ __forceinline__ void targetRadii(const T* h, const float* hf, uint32_
     }
 }
 
-template<class T, bool Stats>
+// Whether the 32 targets of a warp and their search spheres (targets in the order of any lane permutation that leaves
+// lane 0 in place; idle lanes hold the first target) can be folded to one image: offsets from the first target and radii
+// well below half of every period. The same in every kernel that asks: explicit roundings, and maxima.
+template<class T>
+__device__ __forceinline__ bool foldSafe(T xi, T yi, T zi, T r2, const BoxParams<T>& b)
+{
+    const T p[3] = {xi, yi, zi};
+    float e = 0.f, least = INFINITY, r;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+    {
+        T d = RN<T>::sub(p[k], __shfl_sync(0xffffffffu, p[k], 0));
+        if (b.pbc[k])
+        {
+            d     = pbcFoldNb<T>(d, b.pbc[k], b.len[k], b.ilen[k]);
+            least = fminf(least, float(b.len[k]));
+        }
+        e = fmaxf(e, fabsf(float(d)));
+    }
+    if constexpr (std::is_same_v<T, double>) r = __fsqrt_ru(__double2float_ru(r2));
+    else r = __fsqrt_ru(r2);
+    return __fmaf_rn(4.f, warpMaxF(e), __fmul_rn(1.02f, warpMaxF(r))) < __fmul_rn(0.4f, least);
+}
+
+template<class T>
 __global__ void __launch_bounds__(NB_THREADS) findNeighborsKernel(NbArgs<T> a, NbPrep prep)
 {
     constexpr bool F64 = std::is_same_v<T, double>;
@@ -187,9 +212,9 @@ __global__ void __launch_bounds__(NB_THREADS) findNeighborsKernel(NbArgs<T> a, N
                       RN<T>::add(yi, twoh) <= a.b.hi[1] && RN<T>::add(zi, twoh) <= a.b.hi[2];
         pbc = !inside;
     }
-    // in the default mode this kernel only serves warps with a particle whose search sphere crosses a periodic
-    // boundary; findNeighborsGroupKernel serves all others
-    if (a.pathOnlyPbcWarps && !__any_sync(0xffffffffu, active && pbc)) return;
+    // this kernel serves the warps with a particle whose search sphere crosses a periodic boundary that cannot be folded
+    // to one image
+    if (!__any_sync(0xffffffffu, active && pbc) || foldSafe<T>(xi, yi, zi, r2, a.b)) return;
 
     // ---- FP32 pre-filter state (T = double) ----
     float Px = 0, Py = 0, Pz = 0, bx = 0, by = 0, bz = 0, A = 0, Tin = 0, Tout = 0, cLo = 0, cHi = 0;
@@ -228,15 +253,10 @@ __global__ void __launch_bounds__(NB_THREADS) findNeighborsKernel(NbArgs<T> a, N
     const unsigned ngmax = a.ngmax;
     uint32_t* myNb       = a.nb + size_t(i - a.first) * ngmax;
     unsigned nc          = 0;
-    // optional statistics, accumulated per lane and flushed once per warp
-    unsigned long long stCell = 0, stCellExact = 0, stPair = 0, stPairExact = 0, stLeaves = 0, stCand = 0, stNodes = 0;
-
     auto cellTest = [&](int node, unsigned parentMask) -> unsigned {
         bool ok = false;
-        if constexpr (Stats) stNodes++;
         if ((parentMask >> lane) & 1u)
         {
-            if constexpr (Stats) stCell++;
             const T* c = a.centers + 3 * size_t(node);
             const T* s = a.sizes + 3 * size_t(node);
             if constexpr (F64)
@@ -269,7 +289,6 @@ __global__ void __launch_bounds__(NB_THREADS) findNeighborsKernel(NbArgs<T> a, N
                     else if (n2 - E >= cHi) ok = false;
                     else
                     {
-                        if constexpr (Stats) stCellExact++;
                         ok = cellExactF64(xi, yi, zi, false, cellR2, c, s, pa);
                     }
                 }
@@ -284,11 +303,6 @@ __global__ void __launch_bounds__(NB_THREADS) findNeighborsKernel(NbArgs<T> a, N
         uint32_t first = a.layout[leafIdx];
         uint32_t last  = a.layout[leafIdx + 1];
         const bool mine = (mask >> lane) & 1u;
-        if constexpr (Stats)
-        {
-            stLeaves++;
-            stCand += last - first;
-        }
         for (uint32_t base = first; base < last; base += 32)
         {
             uint32_t j = base + lane;
@@ -322,12 +336,10 @@ __global__ void __launch_bounds__(NB_THREADS) findNeighborsKernel(NbArgs<T> a, N
                         {
                             float dx = c.x - bx, dy = c.y - by, dz = c.z - bz;
                             float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                            if constexpr (Stats) stPair++;
                             if (d2 >= Tout) continue;
                             in = d2 < Tin;
                             if (!in)
                             {
-                                if constexpr (Stats) stPairExact++;
                                 in = pairExactF64(xi, yi, zi, false, r2, a.x, a.y, a.z, jj, pa);
                             }
                         }
@@ -384,20 +396,6 @@ __global__ void __launch_bounds__(NB_THREADS) findNeighborsKernel(NbArgs<T> a, N
         }
     }
     if (active) a.nc[i - a.first] = nc;
-    if constexpr (Stats)
-    {
-        unsigned long long v[7] = {stCell, stCellExact, stPair, stPairExact, stLeaves, stCand, stNodes};
-#pragma unroll
-        for (int k = 0; k < 7; ++k)
-        {
-            unsigned long long x = v[k];
-            if (k >= 4) x = lane == 0 ? x : 0; // per-warp quantities: count once
-            for (int o = 16; o > 0; o >>= 1)
-                x += __shfl_xor_sync(0xffffffffu, x, o);
-            if (lane == 0) atomicAdd(a.stats + k, x);
-        }
-        if (lane == 0) atomicAdd(a.stats + 7, 1ull);
-    }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -1287,21 +1285,23 @@ int findNeighbors(cudaStream_t s, const NbArgs<T>& a0, const NbPrep& prep)
     size_t warps  = (size_t(a0.last - a0.first) + 31) / 32;
     size_t blocks = (warps + NB_WARPS - 1) / NB_WARPS;
     NbArgs<T> a   = a0;
-    a.pathOnlyPbcWarps = 0;
     const int G = a.groupSize == 8 || a.groupSize == 16 ? a.groupSize : 32;
     const size_t gwarps = (size_t(a.last - a.first) + G - 1) / G;
     const unsigned gblk = unsigned((gwarps + NB_WARPS - 1) / NB_WARPS);
     if (G == 8) launchGroup<findNeighborsGroupKernel<T, 8>, NBG_MIN_BLOCKS>(gblk, s, a, prep);
     else if (G == 16) launchGroup<findNeighborsGroupKernel<T, 16>, NBG_MIN_BLOCKS>(gblk, s, a, prep);
-    else if (a.stats) launchGroup<findNeighborsTileKernel<T, true>, NT_MIN_BLOCKS>(gblk, s, a, prep);
-    else launchGroup<findNeighborsTileKernel<T, false>, NT_MIN_BLOCKS>(gblk, s, a, prep);
+    else if (a.stats) launchGroup<findNeighborsTileKernel<T, true, false>, NT_MIN_BLOCKS>(gblk, s, a, prep);
+    else launchGroup<findNeighborsTileKernel<T, false, false>, NT_MIN_BLOCKS>(gblk, s, a, prep);
     CSG_CHECK_LAUNCH();
     if (a.anyPbc)
     {
-        // warps with a particle whose search sphere crosses a periodic boundary: per-lane path traversal
-        a.pathOnlyPbcWarps = 1;
-        if (a.stats) findNeighborsKernel<T, true><<<unsigned(blocks), NB_THREADS, 0, s>>>(a, prep);
-        else findNeighborsKernel<T, false><<<unsigned(blocks), NB_THREADS, 0, s>>>(a, prep);
+        // warps with a particle whose search sphere crosses a periodic boundary: folded tiles, or the per-lane path
+        // traversal where the spheres reach too far for one image
+        const unsigned tblk = unsigned((warps + NB_WARPS - 1) / NB_WARPS);
+        if (a.stats) launchGroup<findNeighborsTileKernel<T, true, true>, NT_MIN_BLOCKS>(tblk, s, a, prep);
+        else launchGroup<findNeighborsTileKernel<T, false, true>, NT_MIN_BLOCKS>(tblk, s, a, prep);
+        CSG_CHECK_LAUNCH();
+        findNeighborsKernel<T><<<unsigned(blocks), NB_THREADS, 0, s>>>(a, prep);
         CSG_CHECK_LAUNCH();
     }
     return CS_OK;

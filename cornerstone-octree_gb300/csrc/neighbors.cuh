@@ -24,8 +24,6 @@ struct NbArgs
     uint32_t* nc;
     //! optional traversal statistics of the tile kernel (null: off), listed at its end
     unsigned long long* stats = nullptr;
-    //! path kernel: serve only warps that contain a particle whose search sphere crosses a periodic boundary
-    int pathOnlyPbcWarps = 0;
     //! device error word (may be null): traversal stack overflow of the group kernel
     uint32_t* errWord = nullptr;
     //! smoothing lengths in float with coordinates of type T (then h is unused): the reference's findNeighbors with

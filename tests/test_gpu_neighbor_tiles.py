@@ -12,15 +12,15 @@ from gpu_util import neighbor_lists_equal, to_dev, u32, uniform
 pytestmark = pytest.mark.gpu
 
 
-def _check(cs, O, x, y, z, h, bucket, ngmax, kind=1, bits=64, ext=1.0, lo=None, hi=None):
+def _check(cs, O, x, y, z, h, bucket, ngmax, kind=1, bits=64, ext=1.0, lo=None, hi=None, bnd=0):
     lo = lo if lo is not None else [float(a.min()) - 1e-3 for a in (x, y, z)]
     hi = hi if hi is not None else [float(a.max()) + 1e-3 for a in (x, y, z)]
-    ref = O.pipeline(x, y, z, h, O.make_box(lo, hi), bucket, ngmax, kind, bits, ext)
+    ref = O.pipeline(x, y, z, h, O.make_box(lo, hi, bnd), bucket, ngmax, kind, bits, ext)
     p = cs.Pipeline(64 if x.dtype == np.float64 else 32, bits, kind, bucket, ngmax, ext, 1.0, False, True)
     t = to_dev(x, y, z, h)
     for group in (32, 16):
         p.set_tuning(group, 7)
-        p.run(*t, cs.make_box(lo, hi))
+        p.run(*t, cs.make_box(lo, hi, bnd))
         out = p.outputs()
         torch.cuda.synchronize()
         neighbor_lists_equal(u32(out["neighbors"]).reshape(-1, ngmax), u32(out["neighbor_counts"]), ref["nb"], ref["nc"],
@@ -86,3 +86,21 @@ def test_coarse_keys_and_cell_radii(cs, O, kind, ext):
     x, y, z = (a.astype(np.float32) for a in O.plummer(31, n))
     lo, hi = [float(a.min()) for a in (x, y, z)], [float(a.max()) for a in (x, y, z)]
     _check(cs, O, x, y, z, np.full(n, 0.06, np.float32), 16, 100, kind, 32, ext, lo, hi)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("bnd", [1, (1, 0, 0), (0, 1, 1)])
+@pytest.mark.parametrize("reach", [0.01, 0.05, 0.11, 0.3])
+def test_periodic_boundaries(cs, O, reach, bnd, dtype):
+    """Spheres across faces, edges and corners: folded tiles for the small ones, the path kernel for warps that reach too
+    far for one image, both in the larger ones. A part of the particles sits on the faces."""
+    n = 8000
+    x, y, z = uniform(O, 41, n, -1.0, 2.0, dtype)
+    x[::50], y[7::50], z[9::50], x[11::50] = -1, 2, -1, 2
+    h = (3.0 * reach / 2 * (0.2 + 0.8 * O.philox_uniform(42, 0, n, 0.0, 1.0))).astype(dtype)
+    for kind, bits in ((1, 64), (0, 64)) + (((0, 32),) if dtype == np.float32 else ()):
+        _check(cs, O, x, y, z, h, 16, 300, kind, bits, 1.0, (-1.0,) * 3, (2.0,) * 3, bnd)
+    # a set in the corners of a box far from the origin: the period is large against the radii
+    c = (O.philox_uniform(43, 0, 3 * n, 0.0, 1.0).reshape(3, n) - 0.5) * 0.4
+    x, y, z = (np.where(v < 0, v + 1000.0, v).astype(dtype) for v in c)
+    _check(cs, O, x, y, z, np.full(n, reach * 0.2, dtype), 16, 300, 1, 64, 1.0, (0.0,) * 3, (1000.0,) * 3, bnd)
