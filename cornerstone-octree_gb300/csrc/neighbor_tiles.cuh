@@ -62,7 +62,7 @@ struct TileWarp
     int stack[NT_STACK];
     float4 queue[64];        // kept candidates: frame coordinates and index; a full half becomes fp16 records in place
     uint32_t tileJ[NT_DEFER][32];   // per tile: its candidate indices, the first one last
-    uint32_t mask[NT_DEFER + 1][32]; // per lane: the hits of the tiles that have any (bit 31 - k: candidate k)
+    uint32_t mask[NT_DEFER + 2][32]; // per lane: the hits of the tiles that have any (bit 31 - k: candidate k)
     float4 tgt[32];          // per lane: the target's frame coordinates, its node test radius squared
     float4 thr[32];          // per lane: Tin, Tup, Tsafe
     float4 boxLo[4];         // per sub-group: box of its targets; lo.w: its node test radius squared
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(NB_THREADS, NT_MIN_BLOCKS) findNeighborsTileKe
         int outPend = 0, selfPend = 0; // tiles that may hold outside candidates / the warp's own particles
         int nDefer    = 0;             // tiles whose hits are not yet written
         unsigned held = 0;             // this lane's hits in them,
-        unsigned tileOf = 0;           // the masks that hold them
+        unsigned tileOf = 0;          // the masks that hold them
         int words       = 0;
         for (;;)
         {
@@ -816,18 +816,19 @@ __global__ void __launch_bounds__(NB_THREADS, NT_MIN_BLOCKS) findNeighborsTileKe
                 const uint32_t* mt = &w.mask[0][lane];
                 const uint32_t* jt = w.tileJ[tileOf & 15u];
                 uint32_t m         = *mt;
+                // selects instead of a branch (some lane ends a word in nearly every round), the next word read ahead
+                uint32_t nx = mt[32];
                 while (left > 0)
                 {
                     const int k = 31 - __clz(m);
                     *p          = jt[k];
                     m ^= 1u << k;
-                    if (m == 0u)
-                    {
-                        mt += 32;
-                        m = *mt;
-                        tileOf >>= 4;
-                        jt = w.tileJ[tileOf & 15u];
-                    }
+                    const bool z = m == 0u;
+                    mt += z ? 32 : 0;
+                    m = z ? nx : m;
+                    tileOf >>= z ? 4 : 0;
+                    jt = w.tileJ[tileOf & 15u];
+                    nx = mt[32];
                     ++p;
                     --left;
                 }
