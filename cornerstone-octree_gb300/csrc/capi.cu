@@ -6,6 +6,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 namespace csg
 {
@@ -34,6 +35,57 @@ int smCount()
         cachedDevice = dev;
     }
     return cachedCount;
+}
+
+// the library's memory pool of each device, made on first use and kept for the life of the process (null: it could not
+// be made)
+static cudaMemPool_t workspacePool(int dev)
+{
+    constexpr int MAX_DEVICES = 64;
+    static std::once_flag made[MAX_DEVICES];
+    static cudaMemPool_t pools[MAX_DEVICES] = {};
+    if (dev < 0 || dev >= MAX_DEVICES) return nullptr;
+    std::call_once(made[dev], [dev] {
+        cudaMemPoolProps props{};
+        props.allocType     = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id   = dev;
+        cudaMemPool_t pool  = nullptr;
+        uint64_t keep       = uint64_t(128) << 20;
+        if (cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+            pools[dev] = pool;
+        else
+            (void)cudaGetLastError();
+    });
+    return pools[dev];
+}
+
+cudaError_t workspaceAlloc(void** p, size_t bytes, cudaStream_t s)
+{
+    int dev                     = -1;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+        cudaGetDevice(&dev) == cudaSuccess)
+    {
+        if (cudaMemPool_t pool = workspacePool(dev))
+        {
+            if (cudaMallocFromPoolAsync(p, bytes, pool, s) == cudaSuccess) return cudaSuccess;
+            (void)cudaGetLastError();
+            workspaceTrim();
+        }
+    }
+    else
+        (void)cudaGetLastError();
+    return cudaMallocAsync(p, bytes, s);
+}
+
+void workspaceTrim()
+{
+    int dev = -1;
+    if (cudaGetDevice(&dev) == cudaSuccess)
+        if (cudaMemPool_t pool = workspacePool(dev)) cudaMemPoolTrimTo(pool, 0);
+    (void)cudaGetLastError();
 }
 
 __global__ void copyWordsKernel(const uint32_t* src, uint32_t* dst, unsigned words)

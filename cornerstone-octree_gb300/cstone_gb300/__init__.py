@@ -507,14 +507,14 @@ class Pipeline:
                    level_range=_wrap(o.octree.level_range, max_level(self.key_bits) + 2, torch.int32),
                    internal_to_leaf=_wrap(o.octree.internal_to_leaf, N, torch.int32),
                    leaf_to_internal=_wrap(o.octree.leaf_to_internal, N, torch.int32),
-                   centers=_wrap(o.centers, 3 * N, tdt).view(N, 3), sizes=_wrap(o.sizes, 3 * N, tdt).view(N, 3),
+                   centers=_wrap(o.centers, (N, 3), tdt), sizes=_wrap(o.sizes, (N, 3), tdt),
                    halo_flags=_wrap(o.halo_flags, N, torch.uint8),
                    neighbor_counts=_wrap(o.neighbor_counts, n, torch.int32))
         if o.neighbors:
-            out["neighbors"] = _wrap(o.neighbors, n * self.cfg.ngmax, torch.int32).view(n, self.cfg.ngmax)
+            out["neighbors"] = _wrap(o.neighbors, (n, self.cfg.ngmax), torch.int32)
         if o.search_centers and r.focus_last > r.focus_first:
-            out["search_centers"] = _wrap(o.search_centers, 3 * L, tdt).view(L, 3)
-            out["search_sizes"] = _wrap(o.search_sizes, 3 * L, tdt).view(L, 3)
+            out["search_centers"] = _wrap(o.search_centers, (L, 3), tdt)
+            out["search_sizes"] = _wrap(o.search_sizes, (L, 3), tdt)
         return out
 
 
@@ -589,10 +589,10 @@ class Batch:
                    set_leaf_begin=_wrap(o.set_leaf_begin, S + 1, torch.int32),
                    set_roots=_wrap(o.set_roots, S, torch.int32), set_offsets=_wrap(o.set_offsets, S + 1, torch.int32),
                    prefixes=_wrap(o.octree.prefixes, N, torch.int64),
-                   centers=_wrap(o.centers, 3 * N, tdt).view(N, 3), sizes=_wrap(o.sizes, 3 * N, tdt).view(N, 3),
+                   centers=_wrap(o.centers, (N, 3), tdt), sizes=_wrap(o.sizes, (N, 3), tdt),
                    neighbor_counts=_wrap(o.neighbor_counts, n, torch.int32))
         if o.neighbors:
-            out["neighbors"] = _wrap(o.neighbors, n * self.cfg.ngmax, torch.int32).view(n, self.cfg.ngmax)
+            out["neighbors"] = _wrap(o.neighbors, (n, self.cfg.ngmax), torch.int32)
         return out
 
 
@@ -677,23 +677,22 @@ class Server:
         self.close()
 
 
-def _wrap(ptr, count, dtype):
-    """non-owning torch view of device memory held by the library"""
-    if count == 0 or not ptr:
-        return torch.empty(0, dtype=dtype, device="cuda")
-    nbytes = count * torch.empty(0, dtype=dtype).element_size()
-    arr = _CudaArray(ptr, nbytes)
-    t = torch.as_tensor(arr, device="cuda").view(torch.uint8)[:nbytes]
-    return t.view(dtype)
+_TYPESTR = {torch.float64: "<f8", torch.float32: "<f4", torch.int64: "<i8", torch.int32: "<i4", torch.uint8: "|u1"}
+
+
+def _wrap(ptr, shape, dtype):
+    """non-owning torch view of device memory held by the library (shape: a count or a tuple)"""
+    shape = shape if isinstance(shape, tuple) else (shape,)
+    if not ptr or 0 in shape:
+        return torch.empty(shape, dtype=dtype, device="cuda")
+    return torch.as_tensor(_CudaArray(ptr, shape, _TYPESTR[dtype]), device="cuda")
 
 
 class _CudaArray:
     """exposes a raw device pointer through __cuda_array_interface__ so torch can view it"""
 
-    def __init__(self, ptr, nbytes):
-        self.__cuda_array_interface__ = {"shape": (nbytes,), "typestr": "|u1", "data": (int(ptr), False),
-                                         "version": 3}
-
+    def __init__(self, ptr, shape, typestr):
+        self.__cuda_array_interface__ = {"shape": shape, "typestr": typestr, "data": (int(ptr), False), "version": 3}
 
 
 # ---------------------------------------------------------------------------------------------------------------
