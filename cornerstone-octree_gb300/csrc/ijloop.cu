@@ -58,6 +58,31 @@ __device__ __forceinline__ T densityW(T d2, T hinv)
 }
 
 template<class T>
+__device__ __forceinline__ T fmaRnT(T a, T b, T c)
+{
+    if constexpr (std::is_same_v<T, double>) return __fma_rn(a, b, c);
+    else return __fmaf_rn(a, b, c);
+}
+
+// densityW without a branch: both forms as one sequence of five operations whose operands are selected (a product is
+// fma(a, b, -0), which rounds and signs as the product does). The lanes of a warp take both forms nearly always, and the
+// FP64 pipe (2 lanes per clock and SM) then runs five operations instead of nine.
+template<class T>
+__device__ __forceinline__ T densityWSelect(T d2, T hinv)
+{
+    using R        = RN<T>;
+    const T nz     = T(-0.0);
+    const T q      = R::mul(sqrtRn<T>(d2), hinv);
+    const T q2     = R::mul(q, q);
+    const bool in  = q < T(1);
+    const T u      = fmaRnT<T>(in ? T(1.5) : T(-1), in ? q2 : q, in ? nz : T(2)); // 1.5 q^2      | t = 2 - q
+    const T v      = fmaRnT<T>(in ? T(-1) : u, u, in ? T(1) : nz);                // 1 - 1.5 q^2  | t t
+    const T s      = fmaRnT<T>(in ? T(0.75) : v, in ? q2 : u, nz);                // 0.75 q^2     | (t t) t
+    const T r      = R::mul(s, in ? q : T(0.25));                                 // (0.75 q^2) q | 0.25 ((t t) t)
+    return in ? R::add(v, r) : r;
+}
+
+template<class T>
 __device__ __forceinline__ T foldRn(T d, int pbc, T len, T ilen)
 {
     return RN<T>::sub(d, RN<T>::mul(RN<T>::mul(T(pbc), len), RN<T>::rint_(RN<T>::mul(d, ilen))));
@@ -330,10 +355,17 @@ __device__ __forceinline__ T fromBits(unsigned long long b)
     else return __uint_as_float(uint32_t(b));
 }
 
+// round to nearest float; a double by integer instructions (splitDouble's high part): the conversions of the j-clusters
+// took a tenth of the FP64 pipe's time
 template<class T>
 __device__ __forceinline__ float toFloatRn(T v)
 {
-    if constexpr (std::is_same_v<T, double>) return __double2float_rn(v);
+    if constexpr (std::is_same_v<T, double>)
+    {
+        float hi, lo;
+        splitDouble(v, hi, lo);
+        return hi;
+    }
     else return v;
 }
 
@@ -408,7 +440,7 @@ __global__ void __launch_bounds__(DC_WARPS * 32) densityClusterKernel(const T* _
                 const uint32_t j = uint32_t(queue[slot][owner]);
                 T dx = R::sub(oxi, __ldg(x + j)), dy = R::sub(oyi, __ldg(y + j)), dz = R::sub(ozi, __ldg(z + j));
                 T d2 = R::add(R::add(R::mul(dx, dx), R::mul(dy, dy)), R::mul(dz, dz));
-                T term = d2 < or2 ? R::mul(__ldg(m + j), densityW<T>(d2, ohinv)) : T(-0.0);
+                T term = d2 < or2 ? R::mul(__ldg(m + j), densityWSelect<T>(d2, ohinv)) : T(-0.0);
                 queue[slot][owner] = toBits<T>(term);
             }
         }
