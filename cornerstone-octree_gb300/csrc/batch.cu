@@ -249,9 +249,7 @@ struct Batch final : BatchBase
         if ((rc = linkWs.ensure(buildLinkWorkspaceBytes<uint64_t>(L)))) return rc;
         cs_octree_view v{L, I, N, prefixes.p, childOffsets.as<int32_t>(), parents.as<int32_t>(),
                          levelRange.as<int32_t>(), i2l.as<int32_t>(), l2i.as<int32_t>()};
-        int prefixBits = std::min(64, 3 * br.maxDepth + 1);
-        if ((rc = buildLink<uint64_t>(s, leaves.as<uint64_t>(), L, v, prefixBits, linkWs.p, linkWs.bytes, err + 1)))
-            return rc;
+        if ((rc = buildLink<uint64_t>(s, leaves.as<uint64_t>(), L, v, linkWs.p, linkWs.bytes))) return rc;
         if ((rc = centers.ensure(3 * size_t(N) * sizeof(T)))) return rc;
         if ((rc = sizes.ensure(3 * size_t(N) * sizeof(T)))) return rc;
         if ((rc = geoCentersBatched<T>(s, prefixes.as<uint64_t>(), N, centers.as<T>(), sizes.as<T>(), boxes, S,

@@ -8,15 +8,11 @@ namespace csg
 template<class K>
 size_t buildLinkWorkspaceBytes(int L);
 
-/*! Link the internal tree of leaves[0..L] into `v`. prefixBits (0 = full key width) limits the radix sort of the
- *  placeholder prefixes to their significant bits (3 * deepest leaf level + 1). errWord: device word for sort
- *  timeouts (nullptr = internal). */
+/*! Link the internal tree of leaves[0..L] into `v`. With Ldev (device leaf count) L is a capacity: every launch covers
+ *  it, the kernels use the device count, and the host needs no synchronisation (graphs). */
 template<class K>
-int buildLink(cudaStream_t s, const K* leaves, int L, const cs_octree_view& v, int prefixBits, void* ws,
-              size_t wsBytes, uint32_t* errWord, const int* Ldev = nullptr);
-
-//! with Ldev (device leaf count) L is a capacity: every launch covers it, the kernels use the device count, the
-//! prefix sort runs over the capacity's node count with padding, and the host needs no synchronisation (graphs)
+int buildLink(cudaStream_t s, const K* leaves, int L, const cs_octree_view& v, void* ws, size_t wsBytes,
+              const int* Ldev = nullptr);
 
 template<class K, class T>
 int geoCenters(cudaStream_t s, const K* prefixes, int N, T* centers, T* sizes, const cs_box& box, int kind,

@@ -351,8 +351,7 @@ struct Pipeline final : PipelineBase
         CSG_CUDA_TRY(rec(ev[ST_LINK]));
         cs_octree_view v{cap, Icap, Ncap, prefixes.p, childOffsets.as<int32_t>(), parents.as<int32_t>(),
                          levelRange.as<int32_t>(), i2l.as<int32_t>(), l2i.as<int32_t>()};
-        if ((rc = buildLink<K>(s, incLeaves[nxt].as<K>(), cap, v, 0, linkWs.p, linkWs.bytes, err + 1, Ldev)))
-            return rc;
+        if ((rc = buildLink<K>(s, incLeaves[nxt].as<K>(), cap, v, linkWs.p, linkWs.bytes, Ldev))) return rc;
         CSG_CUDA_TRY(rec(ev[ST_GEO]));
         if ((rc = geoCenters<K, T>(s, prefixes.as<K>(), Ncap, centers.as<T>(), sizes.as<T>(), box, cfg.sfc_kind,
                                    Ldev)))
@@ -683,8 +682,7 @@ struct Pipeline final : PipelineBase
         if ((rc = linkWs.ensure(buildLinkWorkspaceBytes<K>(L)))) return rc;
         cs_octree_view v{L, I, N, prefixes.p, childOffsets.as<int32_t>(), parents.as<int32_t>(),
                          levelRange.as<int32_t>(), i2l.as<int32_t>(), l2i.as<int32_t>()};
-        int prefixBits = std::min(KB, 3 * br.maxDepth + 1);
-        if ((rc = buildLink<K>(s, leaves.as<K>(), L, v, prefixBits, linkWs.p, linkWs.bytes, err + 1))) return rc;
+        if ((rc = buildLink<K>(s, leaves.as<K>(), L, v, linkWs.p, linkWs.bytes))) return rc;
 
         CSG_CUDA_TRY(cudaEventRecord(ev[ST_GEO], s));
         if ((rc = centers.ensure(3 * size_t(N) * sizeof(T)))) return rc;
