@@ -908,7 +908,7 @@ def main():
     achieved = nb_bytes / (nb_ms * 1e-3) / 1e9
     prof = profile_figures(n)
     sm_mhz = clocks.summary().get("sm_mhz") or 2070.0
-    roofline = {"kernel": "findNeighborsGroupKernel<double>", "bound": "issue", "achieved": round(achieved, 1),
+    roofline = {"kernel": "findNeighborsTileKernel<double>", "bound": "issue", "achieved": round(achieved, 1),
                 "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": round(achieved / peak, 4),
                 "traffic": prof.get("traffic"), "algorithmic_bytes": nb_bytes, "ms": round(nb_ms, 4),
                 "traffic_source": prof.get("source"),
@@ -949,7 +949,7 @@ def main():
                 "tree": {"leaves": res.num_leaves, "nodes": res.num_nodes, "iterations": res.iterations,
                          "max_depth": res.max_depth, "focus_leaves": res.focus_last - res.focus_first},
                 "mean_neighbors": round(mean_nc, 2), "h_converged_frac": float((hnc == K_NEIGHBORS).double().mean())}
-        line["gpu_launches"] = gpu_launches_per_step(res) * args.steps
+        line["gpu_launches"] = gpu_launches_per_step() * args.steps
         print(json.dumps(line), flush=True)
     if world > 1:
         import torch.distributed as dist
@@ -957,14 +957,13 @@ def main():
         dist.destroy_process_group()
 
 
-def gpu_launches_per_step(res):
+def gpu_launches_per_step():
     """kernels this library launches in one pipeline step (memsets and copies not counted): keys 1, sort 1 histogram
-    + 1 scan + one pass per 8 key bits, gather 1, build 1 cooperative + 1 one-warp read of its result, link 1 layout +
-    prefix sort + invert + levelRange + link, geometry 1, halos 3 (search boxes, containment list, traversals),
+    + 1 scan + one pass per 8 key bits, gather 1, build 1 cooperative + 1 one-warp read of its result, link 3 (counts,
+    scan, nodes), geometry 1, halos 7 (search boxes, containment list, five passes over the handed-on walks),
     neighbour node prep 1 + outside-leaf marks 1, neighbours 1 (no periodic axis here)"""
     key_passes = (63 + 7) // 8
-    prefix_passes = (3 * res.max_depth + 1 + 7) // 8
-    return 1 + (2 + key_passes) + 1 + (1 + 1) + (1 + 2 + prefix_passes + 3) + 1 + 3 + 2 + 1
+    return 1 + (2 + key_passes) + 1 + (1 + 1) + 3 + 1 + 7 + 2 + 1
 
 
 if __name__ == "__main__":

@@ -40,7 +40,8 @@ def test_link_at_tile_edges(cs, O, splits, where, bits):
     torch.cuda.synchronize()
     assert np.array_equal(keys_u(o.prefixes), ref.prefixes)
     assert np.array_equal(o.child_offsets[: o.num_nodes].cpu().numpy(), ref.child_offsets)
-    assert np.array_equal(o.parents.cpu().numpy(), ref.parents)
+    groups = (o.num_nodes - 1) // 8  # a single leaf has no sibling group, its one slot is never written
+    assert np.array_equal(o.parents.cpu().numpy()[:groups], ref.parents[:groups])
     assert np.array_equal(o.level_range.cpu().numpy(), ref.level_range)
     assert np.array_equal(o.internal_to_leaf.cpu().numpy(), ref.internal_to_leaf)
     assert np.array_equal(o.leaf_to_internal.cpu().numpy(), ref.leaf_to_internal)
