@@ -32,10 +32,10 @@
 // thresholds Tin and Tup). Those, and warps with a sub-group much larger than its radii or with many expansions, test
 // nodes against the 32 search spheres.
 //
-// What bounds it: instruction issue (60 % of the slots) together with latency (fixed-latency chains, shared memory, L2)
-// at 28 warps per SM; DRAM is at 10 %. 16M FP64 Plummer particles, 100 neighbours: 11.7 ms, where one lane per target
+// What bounds it: instruction issue (62 % of the slots) together with latency (fixed-latency chains, shared memory, L2)
+// at 28 warps per SM; DRAM is at 10 %. 16M FP64 Plummer particles, 100 neighbours: 11.3 ms, where one lane per target
 // with packed FP32 tests (two candidates per instruction, the output loop run per batch) took 17.0 ms; 15.9 against 31
-// thousand warp instructions per 32 targets, of which nodes 4, rounds 5, tiles 3.5, output 3 thousand. 32M uniform FP32
+// thousand warp instructions per 32 targets, of which nodes 3.7, rounds 3.8, tiles 3.8, output 3.9 thousand. 32M uniform FP32
 // particles in a periodic box, 57 neighbours: 18.6 against 28.3 ms. 7 blocks of 4 warps per SM measured best (6: 11.9,
 // 8: 12.0 ms, spilling); hits written after every tile: 14.9 ms, after 4 tiles: 11.9 ms.
 //
@@ -44,18 +44,12 @@
 // NT_WIDE + 28 + 7 * 21 + 8.
 #pragma once
 
-constexpr int NT_WIDE  = 128;
-#ifndef NT_LOOSE_AFTER
-#define NT_LOOSE_AFTER 96
-#endif
-constexpr int NT_STACK = NT_WIDE + 28 + 7 * 21 + 9;
+constexpr int NT_WIDE        = 128;
+constexpr int NT_LOOSE_AFTER = 96; // node expansions
+constexpr int NT_STACK       = NT_WIDE + 28 + 7 * 21 + 9;
 // tiles whose hits are written together
-#ifndef NT_DEFER
-#define NT_DEFER 8
-#endif
-#ifndef NT_MIN_BLOCKS
-#define NT_MIN_BLOCKS 7
-#endif
+constexpr int NT_DEFER      = 8;
+constexpr int NT_MIN_BLOCKS = 7;
 
 struct TileWarp
 {

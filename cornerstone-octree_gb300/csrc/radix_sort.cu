@@ -6,8 +6,8 @@
 // by decoupled look-back, then scatters through shared memory so that global writes are runs of consecutive
 // addresses. Traffic per pass: 2 * (sizeof(K) + 4) bytes per pair; the histogram reads the keys once.
 //
-// What bounds it: latency and issue in equal parts (55 % of the issue slots at 24 warps per SM; a pass moves 2.0 to 2.3
-// TB/s, 30 to 35 % of the copy bandwidth). 16M 64-bit keys 1.68 -> 1.22 ms, 20M 32-bit keys 1.02 -> 0.70 ms with the
+// What bounds it: latency and issue in equal parts (55 % of the issue slots at 24 warps per SM; a pass moves 2.3 to 2.9
+// TB/s, 35 to 42 % of the copy bandwidth). 16M 64-bit keys 1.47 -> 1.15 ms, 20M 32-bit keys 1.02 -> 0.70 ms with the
 // ballots in the ranking (a match instruction per key had bound every pass at 100 cycles each), pipelined counter
 // additions and four keys in flight per thread of the histogram (103 -> 52 us for 20M 32-bit keys).
 //
