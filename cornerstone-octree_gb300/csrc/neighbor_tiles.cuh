@@ -156,8 +156,8 @@ __device__ __noinline__ bool foldPath(FoldTarget<T> f, const BoxParams<T>& b, in
 // long as a target's offset and radius together stay below half a period (foldSafe, with room to spare; the remaining
 // warps go to the path kernel). The folds round at the period's scale: A and the node margin grow by 12 eps L; the pairs
 // in the wider band are decided by the reference's folded expressions. 32M uniform FP32 particles: the 8 % of the warps
-// at the boundary took 5.1 ms lane by lane in the path kernel; 2.8 ms here, and 0.6 ms for the path kernel to find nothing
-// left.
+// at the boundary took 5.1 ms lane by lane in the path kernel; 2.7 ms here, and 0.6 ms for the path kernel, whose few
+// remaining warps (targets on both sides of a jump of the curve) are one chain each.
 template<class T, bool Stats, bool Fold>
 __global__ void __launch_bounds__(NB_THREADS, NT_MIN_BLOCKS) findNeighborsTileKernel(NbArgs<T> a, NbPrep prep)
 {
@@ -178,6 +178,8 @@ __global__ void __launch_bounds__(NB_THREADS, NT_MIN_BLOCKS) findNeighborsTileKe
     const size_t wid   = size_t(blockIdx.x) * NB_WARPS + (tid >> 5);
     const size_t base0 = size_t(a.first) + wid * 32;
     if (base0 >= size_t(a.last)) return;
+    if constexpr (Fold)
+        if (a.nc[base0 - a.first] != NB_DEFERRED) return;
     // lane 4 g + t owns target g + 8 t: the row whose mask the quad transpose hands to it
     const int tau      = (lane >> 2) | ((lane & 3) << 3);
     const size_t i64   = base0 + tau;
@@ -193,12 +195,17 @@ __global__ void __launch_bounds__(NB_THREADS, NT_MIN_BLOCKS) findNeighborsTileKe
                             RN<T>::sub(zi, twoh) >= a.b.lo[2] && RN<T>::add(xi, twoh) <= a.b.hi[0] &&
                             RN<T>::add(yi, twoh) <= a.b.hi[1] && RN<T>::add(zi, twoh) <= a.b.hi[2];
         pbc = !inside;
-        if (__any_sync(ALL, active && pbc) != Fold) return;
+        if constexpr (!Fold)
+            if (__any_sync(ALL, active && pbc))
+            {
+                if (lane == 0) a.nc[base0 - a.first] = NB_DEFERRED;
+                return;
+            }
     }
     float len[3] = {}, ilen[3] = {}, lenMax = 0.f; // Fold: the periods (0: not periodic)
     if constexpr (Fold)
     {
-        if (!foldSafe<T>(xi, yi, zi, r2, a.b)) return; // served by findNeighborsKernel
+        if (!foldSafe<T>(xi, yi, zi, r2, a.b)) return; // stays deferred
 #pragma unroll
         for (int k = 0; k < 3; ++k)
             if (a.b.pbc[k])

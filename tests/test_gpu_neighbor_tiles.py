@@ -104,3 +104,26 @@ def test_periodic_boundaries(cs, O, reach, bnd, dtype):
     c = (O.philox_uniform(43, 0, 3 * n, 0.0, 1.0).reshape(3, n) - 0.5) * 0.4
     x, y, z = (np.where(v < 0, v + 1000.0, v).astype(dtype) for v in c)
     _check(cs, O, x, y, z, np.full(n, reach * 0.2, dtype), 16, 300, 1, 64, 1.0, (0.0,) * 3, (1000.0,) * 3, bnd)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("first,last", [(0, 33), (37, 6990), (1000, 1001), (6999, 7000)])
+@pytest.mark.parametrize("reach", [0.05, 0.3])
+def test_periodic_ranges_with_stale_counts(cs, O, reach, first, last, dtype):
+    """Which blocks of 32 the periodic kernels serve is marked in the counts: ranges that begin and end inside a block,
+    into count arrays full of that mark."""
+    n = 7000
+    x, y, z = uniform(O, 51, n, -1.0, 1.0, dtype)
+    obox, box = O.make_box(-1.0, 1.0, 1), cs.make_box(-1.0, 1.0, 1)
+    ref = O.pipeline(x, y, z, np.full(n, reach, dtype), obox, 16, 1, 1, 64, with_neighbors=False)
+    leaves = torch.from_numpy(ref["leaves"].view(np.int64)).cuda()
+    o = cs.build_octree(leaves)
+    t = to_dev(ref["x"], ref["y"], ref["z"], ref["h"])
+    c, s = cs.geo_centers(o.prefixes, box, t[0].dtype, 1)
+    out = (torch.full((last - first, 100), -1, dtype=torch.int32, device="cuda"),
+           torch.full((last - first,), -1, dtype=torch.int32, device="cuda"))
+    rnb, rnc = O.find_neighbors(ref["x"], ref["y"], ref["z"], ref["h"], first, last, obox, ref["tree"], ref["layout"],
+                                ref["centers"], ref["sizes"], 100)
+    cs.find_neighbors(*t, first, last, box, o, torch.from_numpy(ref["layout"].view(np.int32)).cuda(), c, s, 100, out=out)
+    torch.cuda.synchronize()
+    neighbor_lists_equal(u32(out[0]).reshape(-1, 100), u32(out[1]), rnb, rnc, 100)
