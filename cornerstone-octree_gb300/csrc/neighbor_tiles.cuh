@@ -22,7 +22,9 @@
 //    products exact, the two fp16 parts of a value v within 2^-22 |v|, |a|^2 and |b|^2 rounded in fp32, and the tensor
 //    core's accumulation rounded (possibly truncated) to fp32 after each of 16 terms whose absolute sum is below 2^14:
 //      2 * 2 * 64^2 * 2^-22 + 3 * 2^-24 * 2^12 * 2 + 2^-22 * (2^12 + 2^13) + 16 * 2^-23 * 2^14 < 0.045 < E = 1/16,
-//    so D < 0 proves d2_f < Tin, and D >= W = max(Tup - Tin) + 2 E (scaled) proves d2_f >= Tup. The values between
+//    so D < 0 proves d2_f < Tin, and D >= W = max(Tup - Tin) + 2 E (scaled) proves d2_f >= Tup. |b|^2 - Tin + E is
+//    within 2^12 + E because 0 <= Tin <= Tup (a negative Tin is raised to zero) and every target's sqrt(Tup) is a part
+//    of its sphere's radius; with Tin = 0 a tile accepts no pair and leaves all below Tup undecided. The values between
 //    (about two per warp of 32 targets x 100 neighbours) are tested again in FP32 on the frame coordinates and, where
 //    that cannot decide either, in the reference's arithmetic.
 // 4. Output. Every lane appends its target's hits in ascending candidate order, eight tiles at a time.
@@ -308,6 +310,9 @@ __global__ void __launch_bounds__(NB_THREADS, NT_MIN_BLOCKS) findNeighborsTileKe
                 Tin = __fsub_rd(Tin, 0x1p-146f);
                 Tup = __fadd_ru(Tup, 0x1p-146f);
             }
+            // no distance is below zero: the same decisions, and the tiles' sums stay within their bound (tsafe is far
+            // below zero where the radius is small against kappa)
+            Tin = fmaxf(Tin, 0.f);
             // nodes within the cell radius are visited too where it is the larger one: a particle outside its leaf's
             // box can be within r although the box is not
             const float rad = __fmul_ru(a.ext > 1.f ? fmaxf(rr, __fsqrt_ru(cHi)) : rr, 1.f + 64 * EPS);
