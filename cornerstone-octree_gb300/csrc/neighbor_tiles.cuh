@@ -217,6 +217,8 @@ __global__ void __launch_bounds__(NB_THREADS, NT_MIN_BLOCKS) findNeighborsTileKe
                 lenMax  = fmaxf(lenMax, len[k]);
             }
     }
+    // a target that is not finite (in FP32, the frame's type) has no neighbours and takes no part in the frame
+    const bool live = active && fabsf(float(xi)) < INF && fabsf(float(yi)) < INF && fabsf(float(zi)) < INF;
     auto foldF = [&](float d, int k) { return Fold ? fmaf(-len[k], rintf(d * ilen[k]), d) : d; };
     const FoldTarget<T> ftarget{TargetRef<T>{a.x, a.y, a.z, a.h, a.hf, a.ext, i}, pbc};
     const TargetRef<T> tref = ftarget.t;
@@ -247,7 +249,7 @@ __global__ void __launch_bounds__(NB_THREADS, NT_MIN_BLOCKS) findNeighborsTileKe
     }
     for (;; ++passSet)
     {
-        const bool inPass       = active && (!a.numSets || mySet == passSet);
+        const bool inPass       = live && (!a.numSets || mySet == passSet);
         const unsigned passMask = __ballot_sync(ALL, inPass);
         const int rootNode      = a.numSets ? __ldg(a.setRoots + passSet) : 0;
 

@@ -163,12 +163,13 @@ __device__ __forceinline__ void targetRadii(const T* h, const float* hf, uint32_
 
 // Whether the 32 targets of a warp and their search spheres (targets in the order of any lane permutation that leaves
 // lane 0 in place; idle lanes hold the first target) can be folded to one image: offsets from the first target and radii
-// well below half of every period.
+// well below half of every period. Not where an offset is not finite (the maxima pass over NaN).
 template<class T>
 __device__ __forceinline__ bool foldSafe(T xi, T yi, T zi, T r2, const BoxParams<T>& b)
 {
     const T p[3] = {xi, yi, zi};
     float e = 0.f, least = INFINITY, r;
+    bool finite = true;
 #pragma unroll
     for (int k = 0; k < 3; ++k)
     {
@@ -178,8 +179,10 @@ __device__ __forceinline__ bool foldSafe(T xi, T yi, T zi, T r2, const BoxParams
             d     = pbcFoldNb<T>(d, b.pbc[k], b.len[k], b.ilen[k]);
             least = fminf(least, float(b.len[k]));
         }
-        e = fmaxf(e, fabsf(float(d)));
+        finite = finite && fabsf(float(d)) < INFINITY;
+        e      = fmaxf(e, fabsf(float(d)));
     }
+    if (!__all_sync(0xffffffffu, finite)) return false;
     if constexpr (std::is_same_v<T, double>) r = __fsqrt_ru(__double2float_ru(r2));
     else r = __fsqrt_ru(r2);
     return __fmaf_rn(4.f, warpMaxF(e), __fmul_rn(1.02f, warpMaxF(r))) < __fmul_rn(0.4f, least);
