@@ -301,6 +301,9 @@ __global__ void __launch_bounds__(NB_THREADS, NT_MIN_BLOCKS) findNeighborsTileKe
             }
             else { r2lo = r2hi = r2; cLo = cHi = cellR2; }
             rr = __fsqrt_ru(r2hi);
+            // Fold: a target whose sphere lies inside the box meets everything where it is. Below r - 2 kappa the folded
+            // distance is that one (for particles and leaves in the box, up to its faces' rounding)
+            if (Fold && !pbc) cLo = fminf(cLo, r2lo);
             const float tsafe =
                 __fadd_rd(__fadd_rd(__fmul_rd(cLo, 1.f - RHO), -__fmul_ru(__fmul_ru(4.f, kappa), __fsqrt_ru(cHi))),
                           -__fmul_ru(__fmul_ru(4.f, kappa), kappa));
@@ -768,7 +771,10 @@ __global__ void __launch_bounds__(NB_THREADS, NT_MIN_BLOCKS) findNeighborsTileKe
                         const int node = int(code & 0x7fffffffu);
                         if (pathSafe(node) || path(node))
                         {
-                            for (f = ambM & bits; f;)
+                            // (one outside the periodic box is not where it is folded to)
+                            f = (Fold && !pbc ? inM | ambM : ambM) & bits;
+                            inM &= ~f;
+                            while (f)
                             {
                                 const int k = __clz(f);
                                 f ^= 0x80000000u >> k;
