@@ -647,7 +647,6 @@ __global__ void __launch_bounds__(32 * HALO_WARPS)
 // them together. 51 such leaves of a 120k-particle set walk 83 thousand nodes; on 51 of the GPU's 24 thousand groups
 // that took 1.3 ms, handed on twice depth first 0.47 ms, handed on four times breadth first 0.1 ms.
 constexpr int HALO_PASSES = 5;
-constexpr int HALO_MORE   = 1 << 17; // entries of a later pass's list
 
 struct HaloScratch
 {
@@ -814,12 +813,15 @@ __global__ void __launch_bounds__(32 * HALO_WARPS, 10)
         const bool hand = top > low && steps == budget;
         if (__any_sync(0xffffffffu, hand))
         {
-            int at = 0;
-            if (hand && sub == 0) at = atomicAdd(&scratch.base[2 * pass + 2], top - low);
+            // a full list's length is left alone: every group adds at most one stack to it after that, so it stays far
+            // from the counter's end
+            int at       = HALO_MORE;
+            int* handed  = scratch.base + 2 * pass + 2;
+            if (hand && sub == 0 && haloListOpen(__ldcg(handed))) at = atomicAdd(handed, top - low);
             at = __shfl_sync(0xffffffffu, at, lead);
             if (hand)
             {
-                const int room = max(0, min(top - low, HALO_MORE - at));
+                const int room = haloRoom(at, top - low);
                 top -= room;
                 for (int k = sub; k < room; k += 8)
                     scratch.more[(pass + 1) & 1][at + k] = make_int2(leaf, stack[top + k]);

@@ -24,4 +24,17 @@ int findHalos(cudaStream_t s, const K* prefixes, const int32_t* childOffsets, co
 
 size_t haloScratchInts(size_t numFocus);
 
+//! entries of the list that a pass of the halo walks hands on to the next one
+constexpr int HALO_MORE = 1 << 17;
+
+//! whether a list of this length still takes entries
+__host__ __device__ inline bool haloListOpen(int length) { return length >= 0 && length < HALO_MORE; }
+
+//! how many of `left` entries the list takes from place `at` on
+__host__ __device__ inline int haloRoom(int at, int left)
+{
+    if (!haloListOpen(at)) return 0;
+    return left < HALO_MORE - at ? left : HALO_MORE - at;
+}
+
 } // namespace csg
