@@ -681,9 +681,12 @@ _TYPESTR = {torch.float64: "<f8", torch.float32: "<f4", torch.int64: "<i8", torc
 
 
 def _wrap(ptr, shape, dtype):
-    """non-owning torch view of device memory held by the library (shape: a count or a tuple)"""
+    """non-owning torch view of device memory held by the library (shape: a count or a tuple); an array that the library
+    does not have is a view of no rows"""
     shape = shape if isinstance(shape, tuple) else (shape,)
-    if not ptr or 0 in shape:
+    if not ptr:
+        shape = (0,) + shape[1:]
+    if 0 in shape:
         return torch.empty(shape, dtype=dtype, device="cuda")
     return torch.as_tensor(_CudaArray(ptr, shape, _TYPESTR[dtype]), device="cuda")
 
