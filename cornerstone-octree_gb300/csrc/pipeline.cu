@@ -188,6 +188,14 @@ struct Pipeline final : PipelineBase
         cs_tuning win        = keep;
         float winMs          = 0.f;
         int k                = 0;
+        auto note            = [&](const cs_tuning& c, float mean) {
+            if (k < capacity)
+            {
+                if (tried) tried[k] = c;
+                if (ms) ms[k] = mean;
+            }
+            ++k;
+        };
         // mean device time of one stage [first, last) over reps runs with tuning c
         auto score = [&](const cs_tuning& c, int first, int last, float& mean) -> int {
             tuning    = c;
@@ -202,23 +210,22 @@ struct Pipeline final : PipelineBase
                 acc += t;
             }
             mean = acc / float(std::max(1, reps));
-            if (k < capacity)
-            {
-                if (tried) tried[k] = c;
-                if (ms) ms[k] = mean;
-            }
-            ++k;
+            note(c, mean);
             return CS_OK;
         };
+        // nb_by_target_cost reaches no kernel: the candidates of a group size are one kernel, run once, and share its time
+        float groupMs[33] = {};
         for (cs_tuning c : candidates)
         {
             c.sort_items = keep.sort_items;
             float t      = 0.f;
-            if (int rc = score(c, ST_NEIGHBORS, ST_COUNT, t))
+            if (groupMs[c.nb_group] > 0.f) note(c, t = groupMs[c.nb_group]);
+            else if (int rc = score(c, ST_NEIGHBORS, ST_COUNT, t))
             {
                 tuning = keep;
                 return rc;
             }
+            groupMs[c.nb_group] = t;
             if (k == 1 || t < winMs) win = c, winMs = t;
         }
         float sortWin = 0.f;

@@ -602,11 +602,11 @@ int cs_pipeline_set_tuning(cs_pipeline p, const cs_tuning* tuning);
 int cs_pipeline_get_tuning(cs_pipeline p, cs_tuning* tuning);
 /* Autotuner: reruns the inputs of the last cs_pipeline_run / cs_pipeline_run_host, when no cs_pipeline_step came
  * after it (device input arrays must still be valid), reps times for each candidate tuning: first the traversal
- * ({32, 7}, {32, 0}, {32, 5}, {32, 10}, {16, 7}, {8, 7}, scored by the mean device time of the neighbour stage), then,
- * with the fastest of those, the sort's tile shapes (16 and 12 keys per thread, scored by the sort stage). Keeps the
- * fastest as the pipeline's tuning. Writes the best, and up to capacity candidates with their mean ms of the stage
- * that scored them (tried / ms may be NULL); *count = candidates run (8). The outputs afterwards are those of the
- * last candidate's run (identical for every tuning). */
+ * ({32, 7}, {32, 0}, {32, 5}, {32, 10}, {16, 7}, {8, 7}, scored by the mean device time of the neighbour stage; those
+ * of one nb_group are one kernel, run once, and share its time), then, with the fastest of those, the sort's tile shapes
+ * (16 and 12 keys per thread, scored by the sort stage). Keeps the fastest as the pipeline's tuning. Writes the best,
+ * and up to capacity candidates with their mean ms of the stage that scored them (tried / ms may be NULL); *count =
+ * candidates scored (8). The outputs afterwards are those of the last candidate's run (identical for every tuning). */
 int cs_pipeline_autotune(cs_pipeline p, cs_stream_t stream, int reps, cs_tuning* best, cs_tuning* tried, float* ms,
                          int capacity, int* count);
 
