@@ -595,8 +595,8 @@ struct Pipeline final : PipelineBase
         const int keyBits = 3 * KeyTraits<K>::maxLevel;
         if ((rc = sortWs.ensure(radixSortWorkspaceBytes<K>(n, 0, keyBits)))) return rc;
         if ((rc = errWords.ensure(64))) return rc;
-        // error words [0] sort, [1] link sort, [2] halo stack, [3] neighbour stack; [8] the neighbour search's
-        // coordinate bound (float, atomic max from 0)
+        // error words [0] sort, [1] unused, [2] halo stack, [3] neighbour stack; [8] the neighbour search's coordinate
+        // bound (float, atomic max from 0)
         uint32_t* err = errWords.as<uint32_t>();
         float* cmax   = reinterpret_cast<float*>(err + 8);
         if (outPending) CSG_CUDA_TRY(cudaStreamWaitEvent(s, errCopied, 0)); // the previous copy-back read them

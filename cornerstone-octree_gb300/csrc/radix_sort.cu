@@ -7,7 +7,7 @@
 // addresses. Traffic per pass: 2 * (sizeof(K) + 4) bytes per pair; the histogram reads the keys once.
 //
 // What bounds it: latency and issue in equal parts (55 % of the issue slots at 24 warps per SM; a pass moves 2.3 to 2.9
-// TB/s, 35 to 42 % of the copy bandwidth). 16M 64-bit keys 1.47 -> 1.15 ms, 20M 32-bit keys 1.02 -> 0.70 ms with the
+// TB/s, 34 to 43 % of the measured copy rate). 16M 64-bit keys 1.47 -> 1.15 ms, 20M 32-bit keys 1.02 -> 0.70 ms with the
 // ballots in the ranking (a match instruction per key had bound every pass at 100 cycles each), pipelined counter
 // additions and four keys in flight per thread of the histogram (103 -> 52 us for 20M 32-bit keys).
 //

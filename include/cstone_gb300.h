@@ -586,10 +586,10 @@ int cs_pipeline_graph_replays(cs_pipeline p);
  * nb_group: targets per warp of the neighbour traversal (32: pair tests on tensor-core tiles; 16 or 8: 2 or 4 lanes
  * per target).
  * nb_by_target_cost: accepted and kept for callers that set it; no kernel depends on it any more.
- * sort_items: the key sort's tile shape, keys per thread (16 with 3 blocks of 256 threads per SM, or 12 with 4; 0
- * means 16). Default {32, 7, 16}. Setting a tuning ends a step sequence (the next cs_pipeline_step builds from the
- * root). The reference has no counterpart: its traversal shape is the compile-time TravConfig
- * (traversal/find_neighbors.cuh:29-58), and its sort's tiles are CUB's compile-time policy
+ * sort_items: the key sort's tile shape, keys per thread (16 with 3 blocks of 256 threads per SM for 64-bit keys and 4
+ * for 32-bit ones, or 12 with 4; 0 means 16). Default {32, 7, 16}. Setting a tuning ends a step sequence (the next
+ * cs_pipeline_step builds from the root). The reference has no counterpart: its traversal shape is the compile-time
+ * TravConfig (traversal/find_neighbors.cuh:29-58), and its sort's tiles are CUB's compile-time policy
  * (primitives/primitives_gpu.cu:322-356). */
 typedef struct
 {
